@@ -336,7 +336,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_after();
       const float* st = stats + b * 128 + h * 32;
       // visible iff kv <= q + off  <=>  q_local >= kvi - off - q0
-      const int first_visible = p.causal ? (kvi - causal_off - q0) : 0;
+      // A padded key row (of a last key tile, filled with zeros) is seen by no query: its score 0 against the row's log-sum-exp
+      // overflows when all real scores are far below 0 (or the query sees no key), and 0 * inf would reach dQ
+      const int first_visible = kvi >= p.Sk ? BQ : (p.causal ? kvi - causal_off - q0 : 0);
       // this thread's key column carries its own masked query-row ranges (made local to the sub-tile here)
       int4 b4 = make_int4(0, 0, 0, 0);
       if (kMask && kvi < p.Sk) {

@@ -153,6 +153,57 @@ def test_flash_bwd_shared_key_tiles(causal, B, S, Hq, Hkv, parts, monkeypatch):
     assert (got[0] - got[1]).abs().le(got[0].abs() * 2 ** -7 + 1e-3).all()
 
 
+@pytest.mark.parametrize("Sq,Sk", [(200, 200), (64, 1), (300, 129)])
+def test_flash_bwd_padded_keys_and_low_scores(Sq, Sk):
+    """Scores far below zero against a key tile that is not full: the tile's padded rows must not reach dQ through an overflow."""
+    from paddle_b200.ops import _lib, attention
+    torch.manual_seed(Sq + Sk)
+    q = (torch.randn(1, Sq, 4, 128, device="cuda") * 0.02 + 3.0).to(torch.bfloat16).requires_grad_(True)
+    k = (torch.randn(1, Sk, 2, 128, device="cuda") * 0.02 - 3.0).to(torch.bfloat16).requires_grad_(True)
+    v = torch.randn(1, Sk, 2, 128, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    do = torch.randn(1, Sq, 4, 128, device="cuda").to(torch.bfloat16)
+    scale = 1 / math.sqrt(128)                      # every score is near -9 * 128 * scale = -102
+    attention.flash_attn_func(q, k, v, False, scale).backward(do)
+    _lib.check_status()
+    qf, kf, vf = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    rep = [t.repeat_interleave(2, 2).transpose(1, 2) for t in (kf, vf)]
+    (torch.softmax(qf.transpose(1, 2) @ rep[0].mT * scale, -1) @ rep[1]).transpose(1, 2).backward(do.double())
+    for name, got, want in (("dq", q.grad, qf.grad), ("dk", k.grad, kf.grad), ("dv", v.grad, vf.grad)):
+        # P and dS enter the products in bf16 (2^-9 each) and the sums are of terms of one sign or cancel: |dS| sums to about 2 |dP|,
+        # |k|, |q| = 3, so the rounding of dS alone gives up to 2^-8 * 2 * 12 * 3 * scale for dq and Sq / Sk times that for dk
+        bound = {"dq": 0.03, "dk": 0.03 * max(1, 2 * Sq / Sk), "dv": 2 ** -6 * want.abs().max().item()}[name]
+        assert torch.isfinite(got.float()).all(), name
+        assert (got.double() - want).abs().max().item() <= bound + 1e-2, name
+
+
+@pytest.mark.parametrize("S", [200, 100])
+def test_flashmask_rows_that_see_no_key(S):
+    """Query rows for which every key is masked, without a causal mask and with a key tile that is not full: zero output, zero
+    gradient, nothing passed on to the other rows."""
+    import paddle_b200 as paddle
+    from paddle_b200.ops import _lib
+    torch.manual_seed(S)
+    q, k, v = (torch.randn(2, S, h, 128, device="cuda").to(torch.bfloat16).requires_grad_(True) for h in (4, 2, 2))
+    do = torch.randn(2, S, 4, 128, device="cuda").to(torch.bfloat16)
+    # rows [30, 45) and [S - 20, S) see nothing
+    cols = torch.tensor([30, 45, S - 20, S], dtype=torch.int32, device="cuda")
+    idx = torch.stack([cols[2], cols[3], cols[0], cols[1]]).view(1, 1, 1, 4).expand(2, 1, S, 4).contiguous()
+    o = paddle.nn.functional.flashmask_attention(q, k, v, idx, causal=False)
+    o.backward(do)
+    _lib.check_status()
+    masked = _dense_from_flashmask(idx, S, S, False)
+    dead = masked.all(-1)[0, 0]
+    assert int(dead.sum()) == 35
+    qf, kf, vf = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+    ro = _masked_ref(qf, kf, vf, masked, 1 / math.sqrt(128))
+    ro.backward(do.float())
+    assert (o.float() - ro).abs().max().item() < 3e-2
+    assert q.grad[:, dead].float().abs().max().item() == 0
+    for nm, a, b in (("dq", q.grad, qf.grad), ("dk", k.grad, kf.grad), ("dv", v.grad, vf.grad)):
+        err = (a.float() - b).abs().max().item()
+        assert err <= 3e-2 * b.abs().max().item() + 2e-2, f"{nm}: {err}"
+
+
 def _dense_from_flashmask(idx, sq, sk, causal):
     from paddle_b200.nn.functional.flash_attention import _flashmask_dense
     return _flashmask_dense(idx, sq, sk, causal, idx.device)
