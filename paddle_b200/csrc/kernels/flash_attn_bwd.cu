@@ -66,8 +66,8 @@ struct Params {
   const float* lse;     // [B, Hq, Sq] natural log
   const float* delta;   // [B, Hq, Sq]
   float* dq_acc;        // [B, Sq, Hq, 128], added into
-  int parts;            // CTAs that share the query heads of a group; with more than one dK / dV are added into
-  float *dk_acc, *dv_acc;   // [B, Sk, Hkv, 128] (dK not yet scaled)
+  int parts;            // CTAs that share the query heads of a group; with more than one each writes its own fp32 sums
+  float* dkv_part;      // [parts, 2, B, Sk, Hkv, 128]: dK (not yet scaled) and dV of each part
   int* status;
   const int4* bounds;   // column-sparse mask, as in the forward kernel: [B, mask_heads, Sk] of {lts, lte, uts, ute}
   int mask_heads;
@@ -406,23 +406,27 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // -> TMA store
     if (h == 0 && ok && n_it > 0) ok = mbar_wait_warp(&bars->dkv_full, 0, abort_flag, p.status, 310);
     if (p.parts > 1) {
-      // several CTAs share this key tile: fp32 sums go to memory, each warpgroup takes one of dK / dV
+      // several CTAs share this key tile: each stores its fp32 sums, each warpgroup one of dK / dV; dkv_convert_kernel adds the
+      // parts up in a fixed order, so dK / dV are the same on every run
       if (h == 1 && ok && n_it > 0) ok = mbar_wait_warp(&bars->dkv_full, 0, abort_flag, p.status, 312);
-      if (ok && n_it > 0) {
+      if (ok) {
         tc_fence_after();
-        float* dst = (h == 0 ? p.dk_acc : p.dv_acc) + ((static_cast<size_t>(batch) * p.Sk + min(kvi, p.Sk - 1)) * p.Hkv + kv_head) * D;
+        const size_t kv_rows = static_cast<size_t>(p.B) * p.Sk * p.Hkv;
+        float* dst = p.dkv_part + ((part * 2 + h) * kv_rows + (static_cast<size_t>(batch) * p.Sk + min(kvi, p.Sk - 1)) * p.Hkv + kv_head) * D;
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           uint32_t r[32];
-          tmem_ld_32x32(tmem + lane_base + (h == 0 ? COL_DK : COL_DV) + c * 32, r);
-          tmem_ld_wait();
+          if (n_it > 0) {
+            tmem_ld_32x32(tmem + lane_base + (h == 0 ? COL_DK : COL_DV) + c * 32, r);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = 0u;
+          }
           if (kvi < p.Sk) {
 #pragma unroll
             for (int i = 0; i < 32; i += 4)
-              asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c * 32 + i),
-                           "f"(__uint_as_float(r[i])), "f"(__uint_as_float(r[i + 1])), "f"(__uint_as_float(r[i + 2])),
-                           "f"(__uint_as_float(r[i + 3]))
-                           : "memory");
+              *reinterpret_cast<uint4*>(dst + c * 32 + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
           }
           __syncwarp();
         }
@@ -577,6 +581,32 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict
   }
 }
 
+// dk, dv (blockIdx.y = 0, 1; bf16, token / batch strides) = the sum of the parts in their order; dk is scaled.  A row per
+// 16 threads.
+__global__ void __launch_bounds__(256) dkv_convert_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dk,
+                                                          __nv_bfloat16* __restrict__ dv, int parts, int64_t rows, int S, int H,
+                                                          int64_t dk_tok, int64_t dk_batch, int64_t dv_tok, int64_t dv_batch, float scale) {
+  const int which = blockIdx.y;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 16 + (threadIdx.x >> 4);
+  if (row >= rows) return;
+  const int c = (threadIdx.x & 15) * 8;
+  const float* p = src + (which * rows + row) * D + c;
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int k = 0; k < parts; ++k, p += 2 * rows * D) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+    v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+  }
+  const float f = which == 0 ? scale : 1.f;
+  const int64_t bs = row / H;
+  const int h = static_cast<int>(row - bs * H);
+  const int64_t b = bs / S, s = bs - b * S;
+  __nv_bfloat16* dst = which == 0 ? dk + b * dk_batch + s * dk_tok : dv + b * dv_batch + s * dv_tok;
+  *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(h) * D + c) =
+      make_uint4(pack_bf16x2(v[0] * f, v[1] * f), pack_bf16x2(v[2] * f, v[3] * f), pack_bf16x2(v[4] * f, v[5] * f), pack_bf16x2(v[6] * f, v[7] * f));
+}
+
 static bool make_map_bf16(CUtensorMap* m, const void* ptr, int B, int S, int H, int64_t tok, int64_t batch,
                           uint32_t rows) {
   uint64_t dims[4] = {D, static_cast<uint64_t>(H), static_cast<uint64_t>(S), static_cast<uint64_t>(B)};
@@ -590,20 +620,22 @@ static bool make_map_bf16(CUtensorMap* m, const void* ptr, int B, int S, int H, 
 
 // Number of CTAs that should share a (key tile, kv head): the query heads of a group are walked one after the other, so few kv
 // heads leave the GPU idle or its last wave empty.  Costs in us, measured: 1.45 per 64-row sub-tile, 3 per CTA, and with more than
-// one part the fp32 accumulators of dK / dV (zeroed, added to, converted: 14 bytes per element at 6.6 TB/s, two launches).
-// Without a mask whole waves count; with a causal one the longest walk or the average load.
+// one part the fp32 sums of dK / dV (written and read for each part, converted: 8 parts + 2 bytes per element at 6.6 TB/s, a launch).
+// Without a mask whole waves count; with a causal one the longest walk or the average load.  The sums of the parts take no more
+// memory than the fp32 accumulator of dQ, or 64 MB.  (Added into one accumulator by reductions instead, the same shapes take as long
+// up to S = 4096, S = 8192 H = 16/1 702 instead of 735 us, but dK / dV differed from run to run.)
 PD_EXPORT int pd_flash_attn_bwd_parts(int B, int Sq, int Sk, int Hq, int Hkv, int causal) {
   using namespace pd::fab;
   if (B <= 0 || Sq <= 0 || Sk <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0) return 1;
   const int group = Hq / Hkv;
   const double sms = pd::sm_count(), units = static_cast<double>(B) * Hkv * ((Sk + BKV - 1) / BKV), n_sub = (Sq + BQ - 1) / BQ;
-  const double extra = 14.0 * 2 * B * Sk * Hkv * D / 6.6e6 + 6.0;
+  const double kv_elems = 2.0 * B * Sk * Hkv * D, most = fmax(4.0 * B * Sq * Hq * D, 64e6);
   int best = 1;
   double best_cost = 0;
   for (int parts = 1; parts <= group; ++parts) {
-    if (group % parts != 0) continue;
+    if (group % parts != 0 || (parts > 1 && 4.0 * kv_elems * parts > most)) continue;
     const double walk = 1.45 * n_sub * group / parts + 3.0, waves = units * parts / sms;
-    const double cost = walk * (causal ? fmax(1.0, 0.5 * waves) : ceil(waves)) + (parts > 1 ? extra : 0.0);
+    const double cost = walk * (causal ? fmax(1.0, 0.5 * waves) : ceil(waves)) + (parts > 1 ? (8.0 * parts + 2) * kv_elems / 6.6e6 + 6.0 : 0.0);
     if (parts == 1 || cost < 0.97 * best_cost) {
       best = parts;
       best_cost = cost;
@@ -612,11 +644,11 @@ PD_EXPORT int pd_flash_attn_bwd_parts(int B, int Sq, int Sk, int Hq, int Hkv, in
   return best;
 }
 
-// dkv_acc: null, or zero-initialised fp32 [2, B, Sk, Hkv, 128] for `parts` (a divisor of Hq / Hkv) > 1 CTAs per key tile.
+// dkv_part: null, or fp32 scratch [parts, 2, B, Sk, Hkv, 128] for `parts` (a divisor of Hq / Hkv) > 1 CTAs per key tile.
 // dq_acc: zero-initialised fp32 [B, Sq, Hq, 128] (contiguous); delta: fp32 [B, Hq, Sq] scratch;
 // dq/dk/dv: bf16 outputs [B, S, H, 128] with their own token / batch strides (e.g. views of a packed dqkv).  
 PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, const void* v, const void* o,
-                                const float* lse, float* delta, float* dq_acc, float* dkv_acc, void* dq, void* dk,
+                                const float* lse, float* delta, float* dq_acc, float* dkv_part, void* dq, void* dk,
                                 void* dv, int B, int Sq, int Sk, int Hq, int Hkv, int64_t q_tok, int64_t q_batch,
                                 int64_t k_tok, int64_t k_batch, int64_t v_tok, int64_t v_batch, int64_t o_tok,
                                 int64_t o_batch, int64_t do_tok, int64_t do_batch, int64_t dq_tok, int64_t dq_batch,
@@ -626,8 +658,8 @@ PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, c
   using namespace pd;
   using namespace pd::fab;
   if (B <= 0 || Sq <= 0 || Sk <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0) return kErrBadShape;
-  if (parts < 1 || (Hq / Hkv) % parts != 0 || (parts > 1 && dkv_acc == nullptr)) return kErrBadShape;
-  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(d_o) || !aligned16(dkv_acc)) return kErrAlignment;
+  if (parts < 1 || (Hq / Hkv) % parts != 0 || (parts > 1 && dkv_part == nullptr)) return kErrBadShape;
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(d_o) || !aligned16(dkv_part)) return kErrAlignment;
   if ((q_tok % 8) || (k_tok % 8) || (v_tok % 8) || (o_tok % 8) || (do_tok % 8)) return kErrAlignment;
   CUtensorMap tmQ, tmDO, tmK, tmV, tmDK, tmDV;
   bool ok = make_map_bf16(&tmQ, q, B, Sq, Hq, q_tok, q_batch, BQ) &&
@@ -649,8 +681,7 @@ PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, c
       (const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, rows, Sq, Hq, o_tok, o_batch, do_tok, do_batch);
   if (bounds != nullptr && (mask_heads != 1 && mask_heads != Hq && mask_heads != Hkv)) return kErrBadShape;
   if (bounds != nullptr && (!aligned16(bounds) || tile_bounds == nullptr || !aligned16(tile_bounds))) return kErrAlignment;
-  Params p{B, Sq, Sk, Hq, Hkv, causal, scale, scale * 1.4426950408889634f, lse, delta, dq_acc, parts, dkv_acc,
-           dkv_acc == nullptr ? nullptr : dkv_acc + static_cast<size_t>(B) * Sk * Hkv * D, status,
+  Params p{B, Sq, Sk, Hq, Hkv, causal, scale, scale * 1.4426950408889634f, lse, delta, dq_acc, parts, dkv_part, status,
            static_cast<const int4*>(bounds), mask_heads, static_cast<const int4*>(tile_bounds)};
   // kv heads whose operands (q, dO in bf16, dQ in fp32; k, v) share the L2: about 48 MB of them
   const int64_t head_bytes = static_cast<int64_t>(Sq) * (Hq / Hkv) * D * 8 + static_cast<int64_t>(Sk) * D * 4;
@@ -669,9 +700,8 @@ PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, c
                                                                                  dq_batch, scale);
   if (parts > 1) {
     const int64_t kv_rows = static_cast<int64_t>(B) * Sk * Hkv;
-    const unsigned kv_blocks = static_cast<unsigned>((kv_rows + 31) / 32);
-    dq_convert_kernel<<<kv_blocks, 256, 0, stream>>>(p.dk_acc, (__nv_bfloat16*)dk, kv_rows, Sk, Hkv, dk_tok, dk_batch, scale);
-    dq_convert_kernel<<<kv_blocks, 256, 0, stream>>>(p.dv_acc, (__nv_bfloat16*)dv, kv_rows, Sk, Hkv, dv_tok, dv_batch, 1.f);
+    dkv_convert_kernel<<<dim3(static_cast<unsigned>((kv_rows + 15) / 16), 2), 256, 0, stream>>>(
+        dkv_part, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, parts, kv_rows, Sk, Hkv, dk_tok, dk_batch, dv_tok, dv_batch, scale);
   }
   return cudaGetLastError() == cudaSuccess ? kLaunchOk : kErrCuda;
 }

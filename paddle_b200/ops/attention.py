@@ -81,14 +81,14 @@ def bwd(do, q, k, v, o, lse, causal, scale, dq=None, dk=None, dv=None, mask=None
     dk = torch.empty((B, Sk, Hkv, D), dtype=torch.bfloat16, device=dev) if dk is None else dk
     dv = torch.empty((B, Sk, Hkv, D), dtype=torch.bfloat16, device=dev) if dv is None else dv
     assert _view_ok(dq) and _view_ok(dk) and _view_ok(dv)
-    # fp32 accumulators: dq, and dk / dv when several CTAs share a key tile (few kv heads); zeroed together
+    # fp32 accumulator of dq, and the sums of dk / dv of each CTA when several share a key tile (few kv heads)
     parts = _lib.kernels().pd_flash_attn_bwd_parts(B, Sq, Sk, Hq, Hkv, 1 if causal else 0)
-    n_dq = B * Sq * Hq * D
-    dq_acc = torch.zeros(n_dq + (2 * B * Sk * Hkv * D if parts > 1 else 0), dtype=torch.float32, device=dev)
+    dq_acc = torch.zeros(B * Sq * Hq * D, dtype=torch.float32, device=dev)
+    dkv_part = torch.empty(parts * 2 * B * Sk * Hkv * D, dtype=torch.float32, device=dev) if parts > 1 else None
     delta = torch.empty((B, Hq, Sq), dtype=torch.float32, device=dev)
     rc = _lib.kernels().pd_flash_attn_bwd(
         addr(do), addr(q), addr(k), addr(v), addr(o), addr(lse), addr(delta), addr(dq_acc),
-        addr(dq_acc[n_dq:] if parts > 1 else None), addr(dq), addr(dk),
+        addr(dkv_part), addr(dq), addr(dk),
         addr(dv), B, Sq, Sk, Hq, Hkv,
         q.stride(1), q.stride(0), k.stride(1), k.stride(0),
         v.stride(1), v.stride(0), o.stride(1), o.stride(0),
@@ -97,7 +97,7 @@ def bwd(do, q, k, v, o, lse, causal, scale, dq=None, dk=None, dv=None, mask=None
         scale, 1 if causal else 0, addr(mask[0] if mask else None), addr(mask[1] if mask else None),
         mask[0].shape[1] if mask else 0, parts, addr(_lib.status_buffer(dev)), raw_stream())
     check(rc, "pd_flash_attn_bwd")
-    native._count(3 if parts == 1 else 5)
+    native._count(3 if parts == 1 else 4)
     return dq, dk, dv
 
 

@@ -153,6 +153,49 @@ def test_flash_bwd_shared_key_tiles(causal, B, S, Hq, Hkv, parts, monkeypatch):
     assert (got[0] - got[1]).abs().le(got[0].abs() * 2 ** -7 + 1e-3).all()
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 1024, 8, 2), (2, 1999, 32, 8), (1, 777, 40, 5)])
+def test_flash_bwd_dk_dv_repeat_bit_for_bit(causal, B, S, Hq, Hkv):
+    """dK / dV come out the same on every run, also where several CTAs share a key tile."""
+    from paddle_b200.ops import _lib, attention
+    torch.manual_seed(S)
+    q, k, v, do = (torch.randn(B, S, h, 128, device="cuda").to(torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    o, lse = attention.fwd(q, k, v, causal, 0.088)
+    _, dk, dv = attention.bwd(do, q, k, v, o, lse, causal, 0.088)
+    for _ in range(8):
+        _, dk2, dv2 = attention.bwd(do, q, k, v, o, lse, causal, 0.088)
+        assert torch.equal(dk, dk2) and torch.equal(dv, dv2)
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("parts", [1, 2, 4])
+def test_flash_bwd_shared_key_tile_that_no_query_sees(parts, monkeypatch):
+    """Keys hidden from all queries by a column-sparse mask: their CTAs have nothing to walk over and leave zeros, whatever their
+    scratch held."""
+    from paddle_b200.ops import _lib, attention
+    B, S, Hq, Hkv = 1, 300, 4, 1
+    torch.manual_seed(parts)
+    q, k, v, do = (torch.randn(B, S, h, 128, device="cuda").to(torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    idx = torch.full((B, 1, S, 1), S, dtype=torch.int32, device="cuda")
+    idx[:, :, 128:256] = 0                             # the second key tile
+    mask = attention.normalize_flashmask(idx, True, S)
+    o, lse = attention.fwd(q, k, v, True, 0.088, mask)
+    k_ = _lib.kernels()
+
+    class Forced:
+        def __getattr__(self, name):
+            return (lambda *a: parts) if name == "pd_flash_attn_bwd_parts" else getattr(k_, name)
+    monkeypatch.setattr(_lib, "kernels", lambda: Forced())
+    junk = torch.full((8 * B * S * Hkv * 128,), float("nan"), device="cuda")
+    del junk
+    dq, dk, dv = attention.bwd(do, q, k, v, o, lse, True, 0.088, mask=mask)
+    monkeypatch.undo()
+    _lib.check_status()
+    assert all(torch.isfinite(t.float()).all() for t in (dq, dk, dv))
+    assert dk[:, 128:256].abs().max().item() == 0 and dv[:, 128:256].abs().max().item() == 0
+    assert dk[:, :128].abs().max().item() > 0 and dv[:, 256:].abs().max().item() > 0
+
+
 @pytest.mark.parametrize("Sq,Sk", [(200, 200), (64, 1), (300, 129)])
 def test_flash_bwd_padded_keys_and_low_scores(Sq, Sk):
     """Scores far below zero against a key tile that is not full: the tile's padded rows must not reach dQ through an overflow."""
