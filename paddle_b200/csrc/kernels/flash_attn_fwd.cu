@@ -11,15 +11,16 @@
 //
 // Keys are loaded 128 at a time and worked on 64 at a time: a query tile has two 64-column score buffers, so the scores of
 // step u + 1 are in TMEM before the softmax of step u ends.  P(u) is written over S(u); the MMAs of a tile are issued in the order
-//   QK(0) QK(1) | PV(0) QK(2) | PV(1) QK(3) | ...
+//   QK(0, 1) | PV(0) QK(2) | PV(1) QK(3) | ...
+// The first two steps are one product and one softmax step of 128 keys: the row's first reference point is the maximum of both.
 // with one MMA warp for each tile, so that the two streams interleave freely.
 // What bounds it: per 64 keys the MMAs of a tile take 640 cycles (8 of 48 for a 64-column S, 4 of 64 for O) and its softmax some
 // 1000 (ten a column, two warps of a scheduler sharing the special-function unit), and every hand-over between them adds a
 // shared-memory round trip of 150 to 200 cycles beside the softmax warps' traffic.  One MMA warp for both tiles ran two steps
 // behind: of 950 cycles a step it spent 240 on waits that were long complete.  With a warp for each tile a pair of steps takes
 // 1480 cycles instead of 1920.  All waits look once before they spin, and the MMA warps stay converged.
-// B=1 S=4096 H=32: 129 us causal, 242 full (1065 / 1140 TFLOP/s; one MMA warp: 142 / 271; one tile per CTA with 128-key steps: 235 /
-// 364); B=8 H=32/8 full 2786 -> 1741 us (1263 TFLOP/s).  Measured without gain: 128-key steps (one score buffer per tile), part of the
+// B=1 S=4096 H=32: 128 us causal, 243 full (1074 / 1131 TFLOP/s; one MMA warp: 142 / 271; one tile per CTA with 128-key steps: 235 /
+// 364); B=8 H=32/8 full 2786 -> 1836 us (1198 TFLOP/s).  Measured without gain: 128-key steps (one score buffer per tile), part of the
 // exponentials as polynomials on the FMA pipe, looking at the next barrier ahead of the MMAs (7 % slower).
 #include <math.h>
 
@@ -228,6 +229,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // ---------------------------------------------------------------- MMA issuers (whole warps, converged), one for each query tile
     if (n_kv > 0) {
       constexpr uint32_t idesc_qk = make_idesc(BQ, BU, false, false);
+      constexpr uint32_t idesc_qk2 = make_idesc(BQ, BKV, false, false);
       constexpr uint32_t idesc_pv = make_idesc(BQ, D, false, true);
       const int t = NT == 1 ? 0 : __shfl_sync(0xffffffffu, warp - kMmaWarp, 0);
       const int n = t == 0 ? n_u[0] : n_u[NT - 1];
@@ -260,10 +262,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         return true;
       };
       if (NT == 1 || n > 0) {
-        ok = mbar_wait_warp(&bars->q_full[t], 0, abort_flag, p.status, 200 + t);
+        // the first two steps in one product of 128 columns (512 cycles, two of 64 take 768)
+        ok = mbar_wait_warp(&bars->q_full[t], 0, abort_flag, p.status, 200 + t) &&
+             mbar_wait_warp(&bars->k_full[0], 0, abort_flag, p.status, 210);
+        if (ok) {
+          tc_fence_after();
 #pragma unroll
-        for (int b = 0; b < SPT; ++b)
-          if (ok && b < n) ok = issue_qk(0, b, b, 0);
+          for (int ks = 0; ks < D / 16; ++ks) {
+            const uint32_t off = ((ks >> 2) * HALF_BYTES + (ks & 3) * 32) >> 4;
+            umma_bf16_ss_if(leader, s_base, q_desc + off, k_desc + off, idesc_qk2, ks != 0 ? 1u : 0u);
+          }
+          umma_commit_if(leader, &bars->s_full[t][0]);
+          if (n > 1) umma_commit_if(leader, &bars->s_full[t][1]);
+          umma_commit_if(leader, &bars->k_empty[0]);
+        }
       } else {
         ok = pass(&bars->k_full[0], &bars->k_empty[0], 0, 240);
       }
@@ -316,25 +328,21 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     float m_used = -INFINITY;
     uint64_t sum[2] = {f32x2(0.f, 0.f), f32x2(0.f, 0.f)};
     bool ok = true;
-#pragma unroll 1
-    for (int u = 0; u < n_t; ++u) {
-      const int b = u % SPT;
-      if (!mbar_wait_warp(&bars->s_full[t][b], (u / SPT) & 1, abort_flag, p.status, 300 + t)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t s_tmem = tmem + lane_base + COL_S + t * 128 + b * BU;
+    // the scores of step u from TMEM; hidden keys become -inf, which contributes exp2(-inf) = 0
+    auto load_scores = [&](int u, uint32_t (&r)[BU / 32][32]) {
+#pragma unroll
+      for (int c = 0; c < BU / 32; ++c) tmem_ld_32x32(tmem + lane_base + COL_S + t * 128 + (u % SPT) * BU + c * 32, r[c]);
+    };
+    auto hide = [&](int u, uint32_t (&r)[BU / 32][32]) {
       const int col0 = jbase * BKV + u * BU;       // first key column of this step
       int col_limit = p.Sk - 1 - col0;             // highest visible key column (local to this step) for this row
       if (p.causal) col_limit = min(col_limit, qi + causal_off - col0);
-      uint32_t r[BU / 32][32];
-#pragma unroll
-      for (int c = 0; c < BU / 32; ++c) tmem_ld_32x32(s_tmem + c * 32, r[c]);
-      tmem_ld_wait();
       if (__any_sync(0xffffffffu, col_limit < BU - 1)) {
 #pragma unroll
         for (int c = 0; c < BU / 32; ++c) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            if (c * 32 + i > col_limit) r[c][i] = 0xff800000u;   // -inf: contributes exp2(-inf) = 0
+            if (c * 32 + i > col_limit) r[c][i] = 0xff800000u;
           }
         }
       }
@@ -354,7 +362,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       }
-      // row maximum in four chains of three-operand maxima
+    };
+    // row maximum in four chains of three-operand maxima
+    auto row_max = [&](const uint32_t (&r)[BU / 32][32]) {
       float mxs[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -363,7 +373,53 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int i = 2; i < BU / 4; i += 2) mxs[c] = max3(mxs[c], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
       }
-      const float mx = fmaxf(max3(mxs[0], mxs[1], mxs[2]), mxs[3]);
+      return fmaxf(max3(mxs[0], mxs[1], mxs[2]), mxs[3]);
+    };
+    // probabilities of step u over its scores
+    auto write_probs = [&](int u, const uint32_t (&r)[BU / 32][32]) {
+      const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
+      const uint64_t neg_m2 = f32x2(-m_eff, -m_eff);
+#pragma unroll
+      for (int c = 0; c < BU / 32; ++c) {
+        uint32_t pk[16];
+        probs32(r[c], scale2, neg_m2, sum, pk);
+        tmem_st_32x16(tmem + lane_base + COL_S + t * 128 + (u % SPT) * BU + c * 16, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      if (NT == 1) mbar_arrive(&bars->p_full[t][u % SPT]);    // one tile alone: 2 % faster without the warp-wide step
+      else mbar_arrive_warp(&bars->p_full[t][u % SPT]);       // two: 128 arrivals one by one hold up the other tile's waits (252 / 241 us)
+    };
+    int u = 0;
+    if (n_t > 1) {
+      // The first reference point is the maximum of 128 keys, not of 64: it stays for most rows, and the closer it is to the
+      // row's maximum, the more of the large probabilities are near 1, which bf16 holds exactly.  Relative error of O against
+      // 64 bits with 64 / 128 keys: S=130 H=40 0.00224 / 0.00217, B=4 S=1024 H=40 causal 0.002055 / 0.002039, S=4096 H=32
+      // causal 0.002111 / 0.002098; time 8.2 / 8.2, 65.6 / 67.6, 122.8 / 126.8 us.
+      ok = mbar_wait_warp(&bars->s_full[t][1], 0, abort_flag, p.status, 302 + t);
+      if (ok) {
+        tc_fence_after();
+        uint32_t r0[BU / 32][32], r1[BU / 32][32];
+        load_scores(0, r0);
+        load_scores(1, r1);
+        tmem_ld_wait();
+        hide(0, r0);
+        hide(1, r1);
+        m_used = fmaxf(row_max(r0), row_max(r1)) * p.scale_log2;
+        write_probs(0, r0);
+        write_probs(1, r1);
+      }
+      u = SPT;
+    }
+#pragma unroll 1
+    for (; u < n_t && ok; ++u) {
+      if (!mbar_wait_warp(&bars->s_full[t][u % SPT], (u / SPT) & 1, abort_flag, p.status, 300 + t)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t r[BU / 32][32];
+      load_scores(u, r);
+      tmem_ld_wait();
+      hide(u, r);
+      const float mx = row_max(r);
       const float m_new = fmaxf(m_used, mx * p.scale_log2);
       // lazy rescale: only when some row of the warp moved its maximum by more than 2^8
       if (__any_sync(0xffffffffu, (u == 0) || (m_new - m_used > 8.f))) {
@@ -388,18 +444,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       }
-      const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
-      const uint64_t neg_m2 = f32x2(-m_eff, -m_eff);
-#pragma unroll
-      for (int c = 0; c < BU / 32; ++c) {
-        uint32_t pk[16];
-        probs32(r[c], scale2, neg_m2, sum, pk);
-        tmem_st_32x16(s_tmem + c * 16, pk);
-      }
-      tmem_st_wait();
-      tc_fence_before();
-      if (NT == 1) mbar_arrive(&bars->p_full[t][b]);    // one tile alone: 2 % faster without the warp-wide step
-      else mbar_arrive_warp(&bars->p_full[t][b]);       // two: 128 arrivals one by one hold up the other tile's waits (252 / 241 us)
+      write_probs(u, r);
     }
     float l0, l1, l2, l3;
     unpack_f32x2(sum[0], l0, l1);

@@ -386,3 +386,31 @@ def test_flash_fwd_unequal_tiles(causal, B, Sq, Sk):
     assert torch.allclose(lse[live], rl[live], rtol=1e-3, atol=2e-3)
     # P and O are rounded to bf16 (2^-9 relative each); |v| stays below 6
     assert (o.float() - ro).abs().max() <= 6 * 2 ** -8 + 1e-3
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("B,H,Sk", [(1, 2, 100), (1, 2, 128), (1, 2, 300), (10, 40, 300)])
+def test_flash_fwd_largest_probability_is_exact(B, H, Sk, masked):
+    """Each row's largest score lies in the second half of the first 128 keys, less than 2^8 above the first 64: its probability is
+    the reference point of the row (1, exact in bf16), so that the output carries one rounding to bf16 and no second one.  One and
+    two query tiles per CTA; with a column-sparse mask a larger score beside it is hidden and must not count."""
+    from paddle_b200.ops import _lib, attention
+    Sq = min(Sk, 257)
+    a = torch.linspace(0.1, 7.4, Sq, device="cuda").to(torch.bfloat16)
+    q, k, v = (torch.zeros(B, s, H, 128, device="cuda", dtype=torch.bfloat16) for s in (Sq, Sk, Sk))
+    q[..., 0] = a[None, :, None]
+    k[:, 64, :, 0] = 8.0                                # log2 of its probability to that of the others: 1.02 a
+    v[:, 64] = 1.0
+    scale, mask = 1 / math.sqrt(128), None
+    if masked:
+        k[:, 70, :, 0] = 8.5
+        idx = torch.full((B, 1, Sk, 2), Sq, dtype=torch.int32, device="cuda")
+        idx[..., 1] = 0
+        idx[:, :, 70] = torch.tensor([0, Sq], dtype=torch.int32, device="cuda")
+        mask = attention.normalize_flashmask(idx, False, Sq)
+    o, _ = attention.fwd(q, k, v, False, scale, mask)
+    _lib.check_status()
+    want = 1 / (1 + (Sk - 1 - int(masked)) * torch.exp(-8 * a.double() * scale))
+    err = ((o.double() - want[None, :, None, None]) / want[None, :, None, None]).abs().max().item()
+    # one rounding to bf16 (8 significand bits: half a step is at most 2^-8 of the value); sums and exponentials are good to 1e-6
+    assert err <= 2 ** -8 * 1.001, err
