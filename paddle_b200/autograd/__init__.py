@@ -80,7 +80,11 @@ def grad(outputs, inputs, grad_outputs=None, retain_graph=None, create_graph=Fal
 
 
 class saved_tensors_hooks(torch.autograd.graph.saved_tensors_hooks):
-    pass
+    """Hooks over the tensors that operators keep for their backward (python/paddle/autograd/saved_tensors_hooks.py:23).
+    ``pack_hook`` is handed a ``paddle.Tensor`` whatever the operator kept."""
+
+    def __init__(self, pack_hook, unpack_hook):
+        super().__init__(lambda t: pack_hook(as_tensor(t)), unpack_hook)
 
 
 def _jac_one(y, x, batch_axis, create_graph=False):

@@ -23,7 +23,7 @@ from ....._core.tensor import as_tensor
 from .....nn.initializer import Normal
 from .....ops import functional as K
 from .....ops import native
-from .....ops._lib import plain_dispatch
+from .....ops._lib import plain_backward, plain_dispatch
 
 
 def _on_gpu(x, w):
@@ -71,9 +71,9 @@ class _GroupedLinearFP8(torch.autograd.Function):
         return y
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dy):
-        x, w, offsets = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dy):
+        x, w, offsets = saved
         dy = dy.contiguous()
         dx = dw = None
         if ctx.needs_input_grad[0]:

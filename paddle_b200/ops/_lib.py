@@ -166,6 +166,19 @@ def plain_dispatch(fn):
     return run
 
 
+def plain_backward(fn):
+    """For ``backward(ctx, saved, *grads)`` of an autograd function: the saved tensors are fetched with the dispatch as the caller
+    has it (an unpack hook of saved-tensor hooks is the caller's code), the rest runs as under :func:`plain_dispatch`."""
+    off = torch._C.DisableTorchFunctionSubclass
+
+    @functools.wraps(fn)
+    def run(ctx, *grads):
+        saved = ctx.saved_tensors
+        with off():
+            return fn(ctx, saved, *grads)
+    return run
+
+
 _LAUNCH_ERRORS = {
     -1: "bad shape", -2: "pointer/stride alignment", -3: "TMA tensor-map encoding failed",
     -4: "CUDA launch error", -5: "size beyond the supported maximum",

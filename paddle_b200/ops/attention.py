@@ -5,7 +5,8 @@ from __future__ import annotations
 import torch
 
 from . import _lib, native
-from ._lib import addr, check, plain_dispatch, raw_stream
+from .._core.tensor import as_tensor
+from ._lib import addr, check, plain_backward, plain_dispatch, raw_stream
 
 
 def supported(q, k, v) -> bool:
@@ -112,9 +113,9 @@ class _FlashAttnFn(torch.autograd.Function):
         return o, lse
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, do, _dlse):
-        q, k, v, o, lse = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, do, _dlse):
+        q, k, v, o, lse = saved
         dq, dk, dv = bwd(do, q, k, v, o, lse, ctx.causal, ctx.scale, mask=ctx.mask)
         return dq, dk, dv, None, None, None
 
@@ -142,14 +143,14 @@ class _RopeAttnPackedFn(torch.autograd.Function):
         native.rope(rot, cos, sin, None, seq_len=S, half_style=True, out=rot)
         q, k, v = qkv[:, :, :hq], qkv[:, :, hq:hq + hkv], qkv[:, :, hq + hkv:]
         o, lse = fwd(q, k, v, causal, scale)
-        ctx.save_for_backward(qkv, o, lse, cos, sin)
+        ctx.save_for_backward(as_tensor(qkv), o, lse, cos, sin)
         ctx.meta = (B, S, hq, hkv, causal, scale)
         return o
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, do):
-        qkv, o, lse, cos, sin = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, do):
+        qkv, o, lse, cos, sin = saved
         B, S, hq, hkv, causal, scale = ctx.meta
         q, k, v = qkv[:, :, :hq], qkv[:, :, hq:hq + hkv], qkv[:, :, hq + hkv:]
         dqkv = torch.empty_like(qkv)

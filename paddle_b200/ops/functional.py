@@ -14,9 +14,15 @@ import torch
 
 from .._core.tensor import as_tensor
 from . import native
-from ._lib import plain_dispatch
+from ._lib import plain_backward, plain_dispatch
 
-_nosub = torch._C.DisableTorchFunctionSubclass      # see _lib.plain_dispatch
+# see _lib.plain_dispatch; never around an `apply`: the pack hooks of saved-tensor hooks run inside it
+_nosub = torch._C.DisableTorchFunctionSubclass
+
+
+def _contiguous(t):
+    return t if t is None or t.is_contiguous() else as_tensor(t.contiguous())
+
 
 _POLICY = "fused"  # "fused": this library's kernels; "baseline": library kernels (cuBLAS etc.)
 
@@ -55,16 +61,16 @@ class _LinearFn(torch.autograd.Function):
             y = native.gemm(x2, weight)
             if bias is not None:
                 y = y + bias
-        ctx.save_for_backward(x2, weight)
+        ctx.save_for_backward(as_tensor(x2), weight)      # what pack hooks see is a paddle.Tensor
         ctx.has_bias = bias is not None
         ctx.x_shape = x.shape
         ctx.weight_ref = weight
         return y.view(*x.shape[:-1], weight.shape[1])
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dy):
-        x2, weight = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dy):
+        x2, weight = saved
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -130,15 +136,15 @@ class _SplitLinearFn(torch.autograd.Function):
         y = native.gemm(x2, weight) if use_native else x2 @ weight
         if bias is not None:
             y = y + bias
-        ctx.save_for_backward(x2, weight)
+        ctx.save_for_backward(as_tensor(x2), weight)
         ctx.use_native, ctx.x_shape = use_native, x.shape
         ctx.weight_ref, ctx.bias_ref = weight, bias
         return y.view(*x.shape[:-1], weight.shape[1])
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dy):
-        x2, weight = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dy):
+        x2, weight = saved
         dy2 = dy.reshape(-1, dy.shape[-1])
         if ctx.use_native and not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -183,8 +189,9 @@ def linear(x, weight, bias=None):
     if WeightGradStore.split and x.dim() >= 2 and weight.dim() == 2 and torch.is_grad_enabled():
         return as_tensor(_SplitLinearFn.apply(x, weight, bias))
     with _nosub():
-        if _native(x) and weight.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and weight.shape[1] % 8 == 0:
-            return as_tensor(_LinearFn.apply(x, weight, bias))
+        native_ok = _native(x) and weight.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and weight.shape[1] % 8 == 0
+    if native_ok:
+        return as_tensor(_LinearFn.apply(x, weight, bias))
     y = torch.matmul(x, weight)
     return y if bias is None else y + bias
 
@@ -198,9 +205,9 @@ class _MatmulFn(torch.autograd.Function):
         return native.gemm(a, b, ta, tb)
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dc):
-        a, b = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dc):
+        a, b = saved
         ta, tb = ctx.ta, ctx.tb
         dc = dc.contiguous()
         da = db = None
@@ -230,6 +237,8 @@ class _RmsNormFn(torch.autograd.Function):
     @plain_dispatch
     def forward(ctx, x, w, eps, residual):
         y, inv, res_out = native.rms_norm_fwd(x, w, eps, residual=residual, want_residual_out=residual is not None)
+        if res_out is not None:
+            res_out = as_tensor(res_out)
         src = res_out if residual is not None else x
         ctx.save_for_backward(src, w, inv)
         ctx.has_res = residual is not None
@@ -237,9 +246,9 @@ class _RmsNormFn(torch.autograd.Function):
         return y, res_out
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dy, dres):
-        src, w, inv = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dy, dres):
+        src, w, inv = saved
         mg = getattr(ctx.w_ref, "main_grad", None)
         dx, dw = native.rms_norm_bwd(dy.contiguous(), src, w, inv,
                                      dx_add=dres.contiguous() if (ctx.has_res and dres is not None) else None,
@@ -257,11 +266,12 @@ class _RmsNormFn(torch.autograd.Function):
 def rms_norm(x, weight, eps=1e-6, residual=None):
     """Returns ``y`` (and the pre-norm sum when ``residual`` is given)."""
     with _nosub():
-        if _native(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
-            xc = x if x.is_contiguous() else x.contiguous()
-            rc = None if residual is None else (residual if residual.is_contiguous() else residual.contiguous())
-            y, res_out = _RmsNormFn.apply(xc, weight, eps, rc)
-            return (as_tensor(y), as_tensor(res_out)) if residual is not None else as_tensor(y)
+        native_ok = _native(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192
+        if native_ok:
+            x, residual = _contiguous(x), _contiguous(residual)
+    if native_ok:
+        y, res_out = _RmsNormFn.apply(x, weight, eps, residual)
+        return (as_tensor(y), as_tensor(res_out)) if residual is not None else as_tensor(y)
     s = x if residual is None else x + residual
     sf = s.float()
     y = (sf * torch.rsqrt(sf.pow(2).mean(-1, keepdim=True) + eps) * weight.float()).to(x.dtype)
@@ -278,9 +288,9 @@ class _LayerNormFn(torch.autograd.Function):
         return y
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dy):
-        x, w, mean, rstd = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dy):
+        x, w, mean, rstd = saved
         dx, dw, db = native.layer_norm_bwd(dy.contiguous(), x, w, mean, rstd)
         return dx, dw.to(w.dtype), (db.to(w.dtype) if ctx.has_bias else None), None
 
@@ -325,9 +335,9 @@ class _RopeFn(torch.autograd.Function):
         return native.rope(x, cos, sin, position_ids, half_style=half_style)
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dy):
-        cos, sin, pid = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dy):
+        cos, sin, pid = saved
         if not (dy.stride(-1) == 1 and dy.stride(-2) == dy.shape[-1]):
             dy = dy.contiguous()
         return native.rope(dy, cos, sin, pid, half_style=ctx.half_style, backward=True), None, None, None, None
@@ -368,9 +378,9 @@ class _SwigluFn(torch.autograd.Function):
         return native.swiglu_fwd(x, y)
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dout):
-        x, y = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dout):
+        x, y = saved
         dx, dy = native.swiglu_bwd(x, y, dout)
         return dx, dy
 
@@ -380,8 +390,11 @@ def swiglu(x, y=None):
     (python/paddle/incubate/nn/functional/swiglu.py:58)."""
     with _nosub():
         F = x.shape[-1] if y is not None else x.shape[-1] // 2
-        if _native(x) and F % 8 == 0:
-            return as_tensor(_SwigluFn.apply(x.contiguous(), None if y is None else y.contiguous()))
+        native_ok = _native(x) and F % 8 == 0
+        if native_ok:
+            x, y = _contiguous(x), _contiguous(y)
+    if native_ok:
+        return as_tensor(_SwigluFn.apply(x, y))
     if y is None:
         x, y = x.chunk(2, -1)
     return torch.nn.functional.silu(x) * y
@@ -401,9 +414,9 @@ class _SoftmaxCEFn(torch.autograd.Function):
         return loss
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dloss):
-        logits, labels, lse = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dloss):
+        logits, labels, lse = saved
         return native.ce_bwd(logits, labels, lse, dloss.contiguous(), 0, ctx.ignore_index), None, None
 
 
@@ -435,9 +448,9 @@ class _EmbeddingFn(torch.autograd.Function):
         return native.embedding_fwd(ids, table, vocab_start)
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dout):
-        (ids,) = ctx.saved_tensors
+    @plain_backward
+    def backward(ctx, saved, dout):
+        (ids,) = saved
         table = ctx.table_ref
         mg = getattr(table, "main_grad", None)
         if mg is not None:
@@ -485,8 +498,8 @@ class _DropoutAddFn(torch.autograd.Function):
         return native.dropout_add(x, y, p, upscale, seed, offset)
 
     @staticmethod
-    @plain_dispatch
-    def backward(ctx, dout):
+    @plain_backward
+    def backward(ctx, saved, dout):
         p, upscale, seed, offset, has_y = ctx.meta
         dout = dout.contiguous()
         dx = native.dropout_add(dout, None, p, upscale, seed, offset) if ctx.needs_input_grad[0] else None
@@ -523,10 +536,10 @@ def _sdpa_reference(q, k, v, causal, scale):
 def flash_attention(q, k, v, causal=False, scale=None):
     """softmax(q k^T * scale + causal mask) v on ``[batch, seq, heads, head_dim]`` tensors
     (python/paddle/nn/functional/flash_attention.py:358).  Returns the output only."""
+    from . import attention
     with _nosub():
         scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
-        if _native(q):
-            from . import attention
-            if attention.supported(q, k, v):
-                return as_tensor(attention.flash_attn_func(q, k, v, causal, scale))
+        native_ok = _native(q) and attention.supported(q, k, v)
+    if native_ok:
+        return as_tensor(attention.flash_attn_func(q, k, v, causal, scale))
     return _sdpa_reference(q, k, v, causal, scale)
