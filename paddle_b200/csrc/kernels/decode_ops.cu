@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(THREADS) paged_decode_attn_kernel(AttnParams p
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_wait();
   pdl_trigger();
-  const int seq_len = p.seq_lens[b] + p.len_offset;
+  const int seq_len = min(p.seq_lens[b] + p.len_offset, p.max_blocks * PAGE);    // a row of the table names no further pages
   const int pages = (seq_len + PAGE - 1) / PAGE;
   const int per = (pages + p.nsplit - 1) / p.nsplit;
   const int p0 = split * per, p1 = min(pages, p0 + per);
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) decode_qkv_prep_kernel(
     int max_blocks, int64_t qkv_stride, int max_pos) {
   const int b = blockIdx.x;
   const int pos = seq_lens[b];
-  if (pos >= max_pos || pos < 0) return;
+  if (pos >= max_pos || pos < 0 || pos / PAGE >= max_blocks) return;
   const int blk = block_table[static_cast<size_t>(b) * max_blocks + pos / PAGE];
   const int slot = pos % PAGE;
   const bf16* row = qkv + static_cast<size_t>(b) * qkv_stride;

@@ -52,7 +52,7 @@ struct Params {
   const float *cos_t, *sin_t;      // [max_pos, 64]
   const int *seq_lens, *block_table;
   __nv_bfloat16 *k_cache, *v_cache;   // [num_blocks, Hkv, 64, 128]
-  int Hq, Hkv, max_blocks, max_pos;
+  int Hq, Hkv, table_stride, pages, max_pos;   // pages: entries of a block-table row
 };
 
 struct Barriers {
@@ -228,7 +228,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       for (int u = rank * NUM_THREADS + threadIdx.x; u < p.M * 8; u += NUM_THREADS * p.splits) {
         const int m = u >> 3, c = (u & 7) * 8;
         const int pos = p.seq_lens[m];
-        if (pos < 0 || pos >= p.max_pos) continue;
+        if (pos < 0 || pos >= p.max_pos || pos / 64 >= p.pages) continue;
         float a[8], b[8];
         reduce8(part, m, c, p.splits, a);
         reduce8(part, m, 64 + c, p.splits, b);
@@ -251,7 +251,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           dst = p.out + (static_cast<size_t>(m) * p.Hq + head) * BN;
         } else {
           const int kvh = (head - p.Hq) % p.Hkv;
-          const int blk = p.block_table[static_cast<size_t>(m) * p.max_blocks + pos / 64];
+          const int blk = p.block_table[static_cast<size_t>(m) * p.table_stride + pos / 64];
           dst = (head < p.Hq + p.Hkv ? p.k_cache : p.v_cache) + ((static_cast<size_t>(blk) * p.Hkv + kvh) * 64 + pos % 64) * BN;
         }
         store8_bf16(dst + c, a);
@@ -347,14 +347,15 @@ PD_EXPORT int pd_gemm_skinny(const void* x, const void* w, void* out, int M, int
 
 // The qkv projection of a decode step with everything that follows it up to the attention: x [M, K] times W [K, (Hq + 2 Hkv) * 128]
 // (+ bias), rotary embedding of the q and k heads at position seq_lens[m] (cos / sin [max_pos, 64] fp32), q to q_out [M, Hq, 128],
-// the new k / v rows into the cache pages that the block table names.  A sequence whose position is outside the table is left out.
+// the new k / v rows into the cache pages that the block table names (`pages` entries a row, rows `table_stride` apart).  A sequence
+// whose position is outside the rotary table or its pages is left out.
 PD_EXPORT int pd_gemm_skinny_qkv(const void* x, const void* w, const void* bias, const float* cos_t, const float* sin_t,
                                  const int* seq_lens, const int* block_table, void* q_out, void* k_cache, void* v_cache, int M,
-                                 int K, int ldx, int ldw, int Hq, int Hkv, int max_blocks, int max_pos, int weights_ready,
+                                 int K, int ldx, int ldw, int Hq, int Hkv, int table_stride, int pages, int max_pos, int weights_ready,
                                  int* status, cudaStream_t stream) {
   using namespace pd;
   using namespace pd::skinny;
-  if (M <= 0 || M > 128 || K <= 0 || (K % 8) || Hq <= 0 || Hkv <= 0 || max_blocks < 1) return kErrBadShape;
+  if (M <= 0 || M > 128 || K <= 0 || (K % 8) || Hq <= 0 || Hkv <= 0 || pages < 1 || table_stride < 1) return kErrBadShape;
   if (!aligned16(x) || !aligned16(w) || !aligned16(bias) || !aligned16(q_out) || !aligned16(k_cache) || !aligned16(v_cache))
     return kErrAlignment;
   if ((ldx % 8) || (ldw % 8)) return kErrAlignment;
@@ -376,7 +377,8 @@ PD_EXPORT int pd_gemm_skinny_qkv(const void* x, const void* w, const void* bias,
   p.v_cache = static_cast<__nv_bfloat16*>(v_cache);
   p.Hq = Hq;
   p.Hkv = Hkv;
-  p.max_blocks = max_blocks;
+  p.table_stride = table_stride;
+  p.pages = pages;
   p.max_pos = max_pos;
 #define PD_SKINNY(MT_) \
   if (MT == MT_) return launch<MT_, kQkv>(tmW, tmX, p, heads, stream);

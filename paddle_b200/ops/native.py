@@ -614,7 +614,7 @@ def gemm_skinny_qkv(x, w, bias, cos, sin, seq_lens, block_table, q_out, k_cache,
     rc = _lib.kernels().pd_gemm_skinny_qkv(
         ptr(x), ptr(w), ptr(bias), ptr(cos), ptr(sin), ptr(seq_lens), ptr(block_table), ptr(q_out), ptr(k_cache), ptr(v_cache),
         c_int(M), c_int(K), c_int(x.stride(0)), c_int(w.stride(0)), c_int(Hq), c_int(Hkv), c_int(block_table.stride(0)),
-        c_int(cos.shape[0]), c_int(1 if weights_ready else 0), ptr(_lib.status_buffer(x.device)), stream())
+        c_int(block_table.shape[1]), c_int(cos.shape[0]), c_int(1 if weights_ready else 0), ptr(_lib.status_buffer(x.device)), stream())
     check(rc, "pd_gemm_skinny_qkv")
     _count()
     return q_out

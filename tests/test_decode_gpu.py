@@ -158,6 +158,42 @@ def test_skinny_qkv_matches_separate_steps(M, Hq, Hkv, K_, with_bias):
         assert torch.equal(a.abs().amax(-1) == 0, b.abs().amax(-1) == 0)     # the same rows and pages are written
 
 
+@pytest.mark.parametrize("fused", [True, False])
+def test_position_beyond_the_pages_is_left_out(fused):
+    """A rotary table that covers more positions than a sequence has pages: a sequence past its pages writes nothing, into no page of
+    another sequence either, and its attention sees the keys of its own pages only."""
+    from paddle_b200.ops import functional as K
+    from paddle_b200.ops import native, _lib
+    torch.manual_seed(3)
+    M, Hq, Hkv, K_, maxb = 4, 4, 2, 256, 4
+    x = torch.randn(M, K_, device="cuda").bfloat16()
+    w = (torch.randn(K_, (Hq + 2 * Hkv) * 128, device="cuda") * 0.05).bfloat16()
+    cos, sin = K.rope_tables(600, 128, 10000.0, torch.device("cuda"), True)
+    c64, s64 = cos[:, :64].contiguous(), sin[:, :64].contiguous()
+    lens = torch.tensor([256, 255, 599, 300], dtype=torch.int32, device="cuda")
+    table = torch.randperm(M * maxb, device="cuda").int().reshape(M, maxb)
+    kc = torch.randn(M * maxb, Hkv, 64, 128, device="cuda").bfloat16()
+    vc, q = torch.randn_like(kc), torch.zeros(M, Hq, 128, device="cuda", dtype=torch.bfloat16)
+    kc0, vc0 = kc.clone(), vc.clone()
+    if fused:
+        wide = torch.full((M, maxb + 3), 10 ** 6, dtype=torch.int32, device="cuda")     # rows of a wider table, no page behind it
+        wide[:, :maxb] = table
+        native.gemm_skinny_qkv(x, w, None, c64, s64, lens, wide[:, :maxb], q, kc, vc, Hq, Hkv)
+    else:
+        native.decode_qkv_prep(native.gemm(x, w), None, c64, s64, lens, table, q, kc, vc, Hq, Hkv)
+    for now, was in ((kc, kc0), (vc, vc0)):
+        changed = (now != was).any(-1).any(1).nonzero().tolist()
+        assert changed == [[int(table[1, 3]), 63]]                 # the last slot of the one sequence that has room
+    assert q[1].abs().max() > 0 and q[[0, 2, 3]].abs().max() == 0
+    q = torch.randn(M, Hq, 128, device="cuda").bfloat16()
+    for nsplit in (1, 3):
+        out = native.paged_decode_attn(q, kc, vc, table, lens, 0.1, nsplit=nsplit, len_offset=1)
+        torch.cuda.synchronize()
+        _lib.check_status()
+        ref = _ref_paged_attn(q.cpu(), kc.cpu(), vc.cpu(), table.cpu(), [256] * 4, 0.1)
+        assert (out.float().cpu() - ref).abs().max() < 2e-2
+
+
 def test_rms_norm_few_rows_matches_many():
     """One CTA per row (few rows) and one warp per row (many) normalise the same rows alike."""
     from paddle_b200.ops import native
