@@ -1,12 +1,13 @@
 // Two-SM (cta_group::2) variant of the persistent bf16 GEMM for sm_100a:  C[M,N] (=|+=) op(A)[M,K] * op(B)[K,N]
 //
-// A cluster of two CTAs (one SM pair) owns a 256 x 256 output tile.  CTA r of the pair loads rows [128 r, 128 r + 128)
-// of the A tile and columns [128 r, 128 r + 128) of the B tile into ITS OWN shared memory (plain per-CTA TMA loads, no
-// cluster multicast), so every k-block costs each SM 32 KB of shared-memory fill instead of the 48 KB of the
-// 128 x 256 single-CTA tile, and the tensor core reads half of B from the partner SM.  One thread of the leader CTA
-// (cluster rank 0; its MMA warp stays converged and predicates the instruction: with a one-lane branch the same tiles took 4 to
-// 12 % longer, 4096 x 11008 x 4096 with B transposed 258 against 228 us) issues tcgen05.mma.cta_group::2 (M = 256, N = 256, K = 16); the accumulator rows 0-127 live in the
-// leader's TMEM, rows 128-255 in the partner's, and each CTA's four epilogue warps drain their own half.
+// A cluster of two CTAs (one SM pair) owns a 256 x TN output tile, TN = 256 or, for products whose tiles all run at once, 128
+// (tile_n below).  CTA r of the pair loads rows [128 r, 128 r + 128) of the A tile and columns [TN / 2 r, TN / 2 (r + 1)) of the
+// B tile into ITS OWN shared memory (plain per-CTA TMA loads, no cluster multicast), so with TN = 256 every k-block costs each SM
+// 32 KB of shared-memory fill (six stages; 24 KB and eight stages with TN = 128) instead of the 48 KB of the 128 x 256
+// single-CTA tile, and the tensor core reads half of B from the partner SM.  One thread of the leader CTA (cluster rank 0; its MMA
+// warp stays converged and predicates the instruction: with a one-lane branch the same tiles took 4 to 12 % longer, 4096 x 11008 x
+// 4096 with B transposed 258 against 228 us) issues tcgen05.mma.cta_group::2 (M = 256, N = TN, K = 16); the accumulator rows
+// 0-127 live in the leader's TMEM, rows 128-255 in the partner's, and each CTA's four epilogue warps drain their own half.
 //
 // Barriers (all waits bounded, see sm100_prims.cuh):
 //   full[s]   leader only, 1 arrival + transaction bytes of BOTH CTAs (the partner's TMA loads complete on the
@@ -391,6 +392,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   if (warp == 5) tmem_dealloc_2cta(tmem_base, TM_COLS);
 }
 
+// CTA pairs that a call may use: all SMs, or as many as the caller leaves it
+static int max_clusters(int max_ctas) {
+  int clusters = sm_count() / 2;
+  if (max_ctas > 0 && clusters > max_ctas / 2) clusters = max_ctas / 2;
+  return clusters < 1 ? 1 : clusters;
+}
+
 template <bool A_MN, bool B_MN, int EPI, int TILE_N>
 static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, int M, int N, int K,
                           int mn3d, int* status, cudaStream_t stream, int max_ctas, int splits,
@@ -402,24 +410,25 @@ static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
     configured = true;
   }
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N) * splits;
-  int clusters = sm_count() / 2;
-  if (max_ctas > 0 && clusters > max_ctas / 2) clusters = max_ctas / 2;
+  int clusters = max_clusters(max_ctas);
   if (clusters > tiles) clusters = tiles;
-  if (clusters < 1) clusters = 1;
   kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(tmA, tmB, tmC, M, N, K, mn3d, splits, status, bias, act);
   return cudaGetLastError() == cudaSuccess ? kLaunchOk : kErrCuda;
 }
 
-// 256 x 128 tiles when even those all run at once: every pair then does half the work of a 256 x 256 tile (us, wide / narrow:
+// 256 x 128 tiles when even those all run at once on the pairs that the call may use: every pair then does half the work of a 256 x 256 tile (us, wide / narrow:
 // 512 x 1024 x 512 15.3 / 13.3, 818 x 616 x 3064 35.8 / 31.7, 200 x 4096 x 4096 34.8 / 29.7).  With more tiles the wide form wins
 // although its last wave is emptier: a 64-deep block of a narrow tile is 256 tensor cycles and costs some 350 (4096^3: 96 / 124;
 // 1000 x 11008 x 4096, 3 waves against 2.5: 84 / 109).
-static bool narrow_tiles(int M, int N, int splits, int clusters) {
-  return static_cast<int64_t>((M + TILE_M - 1) / TILE_M) * ((N + 127) / 128) * splits <= clusters;
+static int tile_n(int M, int N, int splits, int max_ctas) {
+  return static_cast<int64_t>((M + TILE_M - 1) / TILE_M) * ((N + 127) / 128) * splits <= max_clusters(max_ctas) ? 128 : 256;
 }
 
 }  // namespace gemm2
 }  // namespace pd
+
+// Columns of the tiles that pd_gemm_bf16_2cta works in.
+PD_EXPORT int pd_gemm_2cta_tile_n(int M, int N, int splits, int max_ctas) { return pd::gemm2::tile_n(M, N, splits, max_ctas); }
 
 // Same contract as pd_gemm_bf16 / pd_gemm_bf16_splitk (gemm_sm100.cu); splits = 1 for the plain form.
 PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
@@ -437,7 +446,7 @@ PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, in
   }
   if (!aligned16(A) || !aligned16(B) || !aligned16(C)) return kErrAlignment;
   if ((lda % 8) || (ldb % 8) || (epi == kStoreBf16 ? (ldc % 8) : (ldc % 4))) return kErrAlignment;
-  const int TN = narrow_tiles(M, N, splits, sm_count() / 2) ? 128 : 256, BN_HALF = TN / 2;
+  const int TN = tile_n(M, N, splits, max_ctas), BN_HALF = TN / 2;
   CUtensorMap tmA, tmB, tmC;
   bool ok = true;
   int a3d = 0, b3d = 0;
@@ -470,7 +479,7 @@ PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M
   if (swiglu && (bias != nullptr || (N % 16))) return kErrBadShape;
   if (!aligned16(A) || !aligned16(B) || !aligned16(C)) return kErrAlignment;
   if ((lda % 8) || (ldb % 8) || (ldc % 8)) return kErrAlignment;
-  const int TN = !swiglu && narrow_tiles(M, N, 1, sm_count() / 2) ? 128 : 256, BN_HALF = TN / 2;
+  const int TN = swiglu ? 256 : tile_n(M, N, 1, 0), BN_HALF = TN / 2;
   CUtensorMap tmA, tmB, tmC;
   bool ok = true;
   int a3d = 0, b3d = 0;

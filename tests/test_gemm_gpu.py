@@ -133,3 +133,20 @@ def test_narrow_and_wide_tiles(M, N, K_, ta, tb):
     assert (native.gemm_epilogue(a, b, odd, None, ta, tb).double() - pre).abs().le(pre.abs() * 2 ** -8 + 1e-3).all()
     torch.cuda.synchronize()
     _lib.check_status()
+
+
+@pytest.mark.parametrize("max_ctas", [0, 1, 2, 16, 40])
+def test_tile_width_follows_the_ctas_a_call_may_use(max_ctas):
+    """Narrow tiles only where all of them run at once on the CTA pairs that the caller leaves to the product."""
+    from paddle_b200.ops import _lib, native
+    M, N, K_ = 1000, 1160, 264                       # 4 x 10 narrow tiles
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    pairs = max(1, min(pairs, max_ctas // 2)) if max_ctas else pairs
+    assert _lib.kernels().pd_gemm_2cta_tile_n(M, N, 1, max_ctas) == (128 if 40 <= pairs else 256)
+    torch.manual_seed(max_ctas)
+    a, b = torch.randn(M, K_, device="cuda").bfloat16(), torch.randn(K_, N, device="cuda").bfloat16()
+    ref = a.double() @ b.double()
+    got = native.gemm(a, b, max_ctas=max_ctas)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert (got.double() - ref).abs().le(ref.abs() * 2 ** -8 + 1e-3).all()      # fp32 sums of products of size 1, one rounding
