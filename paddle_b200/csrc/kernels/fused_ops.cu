@@ -250,6 +250,8 @@ __global__ void __launch_bounds__(RN_THREADS) rms_norm_fwd_kernel(
 // Persistent over rows so that the dw partials stay in registers: NV vectors of 8 columns per thread, H <= 2048 NV.
 // Bandwidth-bound when enough is in flight: the next row is fetched (packed, 16 registers at H = 4096) before the current
 // one is reduced, since with one row per CTA at a time the block sum left memory idle.  4096 x 4096: 54 us before.
+// With four vectors a thread needs 221 registers, so one CTA per SM: held to 128 for two it spilled them (4096 x 8192 with / without
+// the added gradient 95 / 66 us, now 72 / 65; 4096 x 7168 93 -> 65).
 __device__ __forceinline__ void widen8(const bf16x8& r, float (&f)[8]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -259,7 +261,7 @@ __device__ __forceinline__ void widen8(const bf16x8& r, float (&f)[8]) {
   }
 }
 template <typename WT, int NV>
-__global__ void __launch_bounds__(RN_THREADS, 2) rms_norm_bwd_kernel(
+__global__ void __launch_bounds__(RN_THREADS, NV == 4 ? 1 : 2) rms_norm_bwd_kernel(
     const bf16* __restrict__ dy, const bf16* __restrict__ x, const WT* __restrict__ w,
     const float* __restrict__ inv_rms, bf16* __restrict__ dx, const bf16* __restrict__ dx_add,
     float* __restrict__ dw_partial, int rows, int H) {
