@@ -194,6 +194,20 @@ def test_position_beyond_the_pages_is_left_out(fused):
         assert (out.float().cpu() - ref).abs().max() < 2e-2
 
 
+def test_refused_launch_leaves_no_error_behind():
+    """A launch that the CUDA runtime refuses (2^32 rows give an empty grid) is reported by its own launcher, not by the next one."""
+    from paddle_b200.ops import _lib, native
+    x = torch.randn(4, 8, device="cuda").bfloat16()
+    y, inv = torch.empty_like(x), torch.empty(4, device="cuda")
+    rc = _lib.kernels().pd_rms_norm_fwd(x.data_ptr(), None, x.data_ptr(), 0, y.data_ptr(), None, inv.data_ptr(), 2 ** 32, 8, 1e-5,
+                                        _lib.raw_stream())
+    assert rc == -4
+    g = torch.randn(4, 32, device="cuda").bfloat16()
+    got = native.swiglu_fwd(g).float()
+    a, b = g.float().chunk(2, 1)
+    assert torch.allclose(got, torch.nn.functional.silu(a) * b, rtol=2e-2, atol=1e-2)
+
+
 def test_rms_norm_few_rows_matches_many():
     """One CTA per row (few rows) and one warp per row (many) normalise the same rows alike."""
     from paddle_b200.ops import native
