@@ -233,7 +233,7 @@ class FusedMultiTransformer(Layer):
 
     # ------------------------------------------------------------------ serving path (paged cache, native kernels)
     def prepare_paged(self, tp_group=None, max_batch=64):
-        """Pack weights as ``[in, out]`` bf16 matrices and allocate the decode workspaces."""
+        """Pack weights as ``[in, out]`` bf16 matrices and allocate the decode workspaces that batches of ``max_batch`` need."""
         assert self.norm_type == "rmsnorm" and self.activation == "swiglu" and self.head_dim == 128, \
             "the paged path covers the Llama family: RMSNorm, SwiGLU, head_dim 128"
         E, nh, hkv, hd = self.embed_dim, self.num_heads, self.kv_heads, self.head_dim
@@ -262,12 +262,15 @@ class FusedMultiTransformer(Layer):
         self._ws = {}
         for name, N, Kdim in (("qkv", (nh + 2 * hkv) * hd, E), ("out", E, nh * hd), ("ffn1", 2 * self.dim_ff, E),
                               ("ffn2", E, self.dim_ff)):
-            s = native.suggest_splits(max_batch, N, Kdim) if dev.type == "cuda" else 1
+            # split-K sums are for what the weight-streaming kernel does not take (see _gemm)
+            streams = max_batch <= 128 and all(native.gemm_skinny_weight_ok(P[name]) for P in packed)
+            s = native.suggest_splits(max_batch, N, Kdim) if dev.type == "cuda" and not streams else 1
             self._ws[name] = (s, torch.zeros((max_batch, N), dtype=torch.float32, device=dev) if s > 1 else None)
         return self
 
     def _gemm(self, name, x, w, residual=None):
-        """x [M, K] @ w [K, N] (+ residual); the weight-streaming kernel for the skinny decode shapes."""
+        """x [M, K] @ w [K, N] (+ residual): up to 128 rows of aligned operands in the weight-streaming kernel, other batches up to
+        ``max_batch`` as split-K with an fp32 workspace, the rest as a plain product."""
         from ....ops import native
         M = x.shape[0]
         if native.gemm_skinny_ok(x, w) and (residual is None or native.rows16(residual)):
@@ -345,7 +348,7 @@ class FusedMultiTransformer(Layer):
             wsp = (torch.empty((B, nh, nsplit, 128), dtype=torch.float32, device=x.device),
                    torch.empty((B, nh, nsplit, 2), dtype=torch.float32, device=x.device))
         scale = 1.0 / math.sqrt(128)
-        # the fused projection reads the tables in 16-byte pieces of fp32
+        # the fused projection takes fp32 tables [positions, 64]
         fused_qkv = all(t.dtype == torch.float32 and t.is_contiguous() and t.shape[-1] == 64 for t in (cos64, sin64))
         for i in range(self.num_layers):
             P = self._packed[i]

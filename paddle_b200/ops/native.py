@@ -575,6 +575,11 @@ def gemm_skinny_ok(x, w):
             and x.shape[1] % 8 == 0 and w.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def gemm_skinny_weight_ok(w):
+    """Whether :func:`gemm_skinny_ok` holds for ``w`` with every contiguous bf16 ``x`` of at most 128 rows."""
+    return w.dim() == 2 and w.dtype == BF16 and w.shape[0] % 8 == 0 and w.shape[1] % 8 == 0 and rows16(w)
+
+
 @plain_dispatch
 def gemm_skinny(x, w, bias=None, residual=None, swiglu=False, splits=0, out=None, weights_ready=False):
     """``x @ w (+ bias) (+ residual)`` for at most 128 rows in one kernel that streams the weights (fp32 sums over a cluster

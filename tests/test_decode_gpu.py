@@ -266,6 +266,35 @@ def test_paged_engine_matches_training_forward():
     assert torch.equal(infer.generate(ids, NEW, use_cuda_graph=True), greedy)       # back to greedy re-captures
 
 
+@pytest.mark.parametrize("max_batch", [3, 128, 130])
+def test_projection_workspaces_only_for_larger_batches(max_batch):
+    """Up to 128 rows no projection needs an fp32 workspace; a model prepared for more has one for the rows between, and every batch
+    gives the same product."""
+    import paddle_b200 as paddle
+    from paddle_b200.models.llama import LlamaConfig
+    from paddle_b200.models.llama_infer import LlamaForCausalLMInference
+    from paddle_b200.ops import _lib
+    paddle.set_device("gpu:0")
+    cfg = LlamaConfig.tiny(hidden_size=256, intermediate_size=512, num_attention_heads=2, num_hidden_layers=1,
+                           vocab_size=512, dtype="bfloat16", max_position_embeddings=128)
+    t = LlamaForCausalLMInference(cfg).transformer
+    t.prepare_paged(None, max_batch)
+    sizes = [0 if ws is None else ws.numel() for _, ws in t._ws.values()]
+    assert (sum(sizes) > 0) == (max_batch > 128), sizes
+    w = t._packed[0]["ffn2"]
+    torch.manual_seed(max_batch)
+    with torch.no_grad():
+        w.copy_(torch.randn(w.shape, device="cuda") * 0.05)
+    for M in (1, min(max_batch, 128), max_batch, max_batch + 70):
+        x = torch.randn(M, 512, device="cuda").bfloat16()
+        r = torch.randn(M, 256, device="cuda").bfloat16()
+        want = x.double() @ w.double() + r.double()
+        # one rounding of the result, and of the product before the sum where that is a step of its own
+        assert (t._gemm("ffn2", x, w, residual=r).double() - want).abs().le(want.abs() * 2 ** -8 + 2 ** -6).all(), M
+    torch.cuda.synchronize()
+    _lib.check_status()
+
+
 def test_withheld_signal_returns_status_not_hang():
     """Bounded device-side wait: the fused GEMM->all-reduce kernel is launched as rank 0 of 2 while nothing ever
     plays rank 1 (its slab counter increments go to a dummy array), so the wait on the arrival counter runs out
