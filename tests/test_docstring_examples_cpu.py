@@ -38,9 +38,10 @@ GROUPS = {
 
 @pytest.mark.timeout(900)
 @pytest.mark.parametrize("group", sorted(GROUPS))
-def test_reference_docstring_examples(group):
+def test_reference_docstring_examples(group, tmp_path, monkeypatch):
     import paddle
     from docstring_harness import run_file
+    monkeypatch.chdir(tmp_path)                     # some examples save files by a relative name
     patterns, min_pass, max_bad, *rest = GROUPS[group]
     allow = rest[0] if rest else ()
     files = sorted(f for p in patterns for f in glob.glob(os.path.join(REF, p)))
