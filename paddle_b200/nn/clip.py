@@ -63,7 +63,8 @@ class ClipGradByGlobalNorm(ClipGradBase):
         return torch.stack([g.float().pow(2).sum() for g in grads]).sum().reshape(1)
 
     def clip_coef(self, norm_sq):
-        if norm_sq.is_cuda and norm_sq.dtype == torch.float32 and norm_sq.numel() == 1 and not norm_sq.requires_grad:
+        if norm_sq.is_cuda and norm_sq.dtype == torch.float32 and norm_sq.numel() == 1 and not norm_sq.requires_grad \
+                and norm_sq.get_device() == torch.cuda.current_device():            # the kernel runs on the current device
             from ..ops import native
             return native.clip_coef(norm_sq, float(self.clip_norm))
         gn = norm_sq.sqrt()

@@ -320,3 +320,24 @@ def test_flag_registry_covers_the_reference_and_effects_apply(tmp_path):
     env = dict(os.environ, FLAGS_cudnn_deterministic="1", FLAGS_use_autotune="true", PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     out = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=120).stdout
     assert out.strip() == "True {'FLAGS_use_autotune': True}"
+
+
+def test_clip_factor_on_another_device_is_not_launched_here(monkeypatch):
+    """The one-launch clip factor runs on the current device only; a norm that lives on another GPU takes the element-wise form."""
+    from paddle_b200.nn.clip import ClipGradByGlobalNorm
+    from paddle_b200.ops import native
+
+    class OnGpu1(torch.Tensor):
+        is_cuda = True
+
+        def get_device(self):
+            return 1
+    launched = []
+    monkeypatch.setattr(native, "clip_coef", lambda n, c: launched.append(c))
+    norm_sq = torch.tensor([16.0]).as_subclass(OnGpu1)
+    clip = ClipGradByGlobalNorm(1.0)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    assert float(clip.clip_coef(norm_sq)) == 0.25 and not launched
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    clip.clip_coef(norm_sq)
+    assert launched == [1.0]
