@@ -24,6 +24,15 @@ def _contiguous(t):
     return t if t is None or t.is_contiguous() else as_tensor(t.contiguous())
 
 
+def _like(out, x):
+    """The result of an operator that keeps the shape of ``x``: distributed as ``x`` is."""
+    mesh = getattr(x, "_dist_mesh", None)
+    if mesh is None:
+        return as_tensor(out)
+    from ..distributed.auto_parallel.dist_tensor import DistTensor
+    return DistTensor.wrap(out, mesh, x._dist_placements)
+
+
 _POLICY = "fused"  # "fused": this library's kernels; "baseline": library kernels (cuBLAS etc.)
 
 
@@ -271,7 +280,7 @@ def rms_norm(x, weight, eps=1e-6, residual=None):
             x, residual = _contiguous(x), _contiguous(residual)
     if native_ok:
         y, res_out = _RmsNormFn.apply(x, weight, eps, residual)
-        return (as_tensor(y), as_tensor(res_out)) if residual is not None else as_tensor(y)
+        return (_like(y, x), _like(res_out, x)) if residual is not None else _like(y, x)
     s = x if residual is None else x + residual
     sf = s.float()
     y = (sf * torch.rsqrt(sf.pow(2).mean(-1, keepdim=True) + eps) * weight.float()).to(x.dtype)
@@ -301,7 +310,7 @@ def layer_norm(x, normalized_shape, weight=None, bias=None, eps=1e-5):
             and (isinstance(normalized_shape, int) or len(normalized_shape) == 1)):
         if bias is not None and bias.dtype != weight.dtype:
             bias = bias.to(weight.dtype)
-        return as_tensor(_LayerNormFn.apply(x.contiguous(), weight, bias, eps))
+        return _like(_LayerNormFn.apply(x.contiguous(), weight, bias, eps), x)
     ns = (normalized_shape,) if isinstance(normalized_shape, int) else tuple(normalized_shape)
     return torch.nn.functional.layer_norm(x, ns, weight, bias, eps)
 
@@ -519,7 +528,7 @@ def _native_any(x):
 def dropout_add(x, y, p, upscale=True, seed_offset=None):
     """``dropout(x) + y`` (``y`` may be None) in one kernel; returns ``(out, (seed, offset))``."""
     seed, offset = seed_offset if seed_offset is not None else _next_philox(x.numel())
-    return as_tensor(_DropoutAddFn.apply(x, y, float(p), bool(upscale), int(seed), int(offset))), (seed, offset)
+    return _like(_DropoutAddFn.apply(x, y, float(p), bool(upscale), int(seed), int(offset)), x), (seed, offset)
 
 
 # ------------------------------------------------------------------------------------------- attention

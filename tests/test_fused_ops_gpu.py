@@ -272,3 +272,24 @@ def test_rope_head_dims(D, heads):
             got = native.rope(x, cos, sin, p, half_style=True, backward=back)
             ref = K._rope_torch(x, cos, -sin if back else sin, p, True)
             assert (got.float() - ref.float()).abs().max() <= ref.float().abs().max() * 2 ** -7
+
+
+def test_shape_keeping_operators_keep_the_distribution():
+    """Norms and dropout of a distributed tensor are distributed as their input is."""
+    import paddle_b200 as paddle
+    import paddle_b200.distributed as dist
+    from paddle_b200.ops import functional as K
+    paddle.set_device("gpu:0")
+    mesh = dist.ProcessMesh([0], dim_names=["x"])
+
+    def make(*shape):
+        t = dist.shard_tensor(paddle.to_tensor(torch.randn(shape, device="cuda").bfloat16()), mesh, [dist.Replicate()])
+        t.stop_gradient = False
+        return t
+    x, w = make(2, 8, 256), make(256)
+    outs = [K.rms_norm(x, w), *K.rms_norm(x, w, residual=x), K.layer_norm(x, 256, w, w), K.dropout_add(x, x, 0.1)[0]]
+    for o in outs:
+        assert o.is_dist() and o.process_mesh == mesh and o.placements == [dist.Replicate()] and o.shape == [2, 8, 256]
+    sum(o.sum() for o in outs).backward()
+    assert x.grad is not None and torch.isfinite(x.grad.float()).all()
+    assert not K.rms_norm(paddle.to_tensor(torch.randn(4, 256, device="cuda").bfloat16()), w).is_dist()
