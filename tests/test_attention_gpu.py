@@ -414,3 +414,57 @@ def test_flash_fwd_largest_probability_is_exact(B, H, Sk, masked):
     err = ((o.double() - want[None, :, None, None]) / want[None, :, None, None]).abs().max().item()
     # one rounding to bf16 (8 significand bits: half a step is at most 2^-8 of the value); sums and exponentials are good to 1e-6
     assert err <= 2 ** -8 * 1.001, err
+
+
+def _two_tile_masks(S, B, Hq):
+    """Masks for grids that take two query tiles per CTA: (name, causal, startend_row_indices)."""
+    for name, causal, idx in _flashmask_cases(S, "cpu"):
+        yield name, causal, idx.expand(B, 1, S, idx.shape[-1])
+    # a document mask of its own for every head and sequence
+    g = torch.Generator().manual_seed(S)
+    cut = torch.randint(1, S, (B, Hq, 1), generator=g)
+    cols = torch.arange(S).view(1, 1, S)
+    ends = torch.where(cols < cut, cut, torch.full_like(cut, S)).to(torch.int32)
+    starts = torch.where(cols < cut, torch.zeros_like(cut), cut).to(torch.int32)
+    yield "documents per head", True, ends.unsqueeze(-1)
+    yield "documents per head", False, torch.stack([ends, starts], -1)
+    # rows 128 .. 383 see nothing: the second tile of the first pair and the first tile of the second pair
+    band = torch.tensor([128, 256, 256, 384], dtype=torch.int32)
+    yield "one tile of a pair", False, band.expand(B, 1, S, 4)
+    # the first 128 rows see the last keys only and the others the first keys only, so the tiles of a pair share no key tile
+    half = torch.full((S, 4), S, dtype=torch.int32)
+    half[:S // 2] = torch.tensor([0, 128, 0, 0], dtype=torch.int32)
+    half[S // 2:] = torch.tensor([128, S, 0, 0], dtype=torch.int32)
+    yield "tiles apart", False, half.view(1, 1, S, 4).expand(B, 1, S, 4)
+
+
+@pytest.mark.parametrize("B,S", [(4, 520), (2, 1000)])
+def test_flashmask_two_query_tiles(B, S):
+    """The masked kernels with two query tiles per CTA (enough blocks that the size rule takes them): output, log-sum-exp and gradients
+    against a dense mask, for tiles of a pair that see other keys than each other, or none."""
+    from paddle_b200.ops import _lib, attention
+    Hq, Hkv, scale = 40, 8, 1 / math.sqrt(128)
+    for name, causal, idx in _two_tile_masks(S, B, Hq):
+        idx = idx.cuda().contiguous()
+        torch.manual_seed(S)
+        q, k, v, do = (torch.randn(B, S, h, 128, device="cuda").to(torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+        mask = attention.normalize_flashmask(idx, causal, S)
+        o, lse = attention.fwd(q, k, v, causal, scale, mask)
+        dq, dk, dv = attention.bwd(do, q, k, v, o, lse, causal, scale, mask=mask)
+        _lib.check_status()
+        masked = _dense_from_flashmask(idx, S, S, causal)
+        dead = masked.all(-1).expand(B, Hq, S)
+        qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+        ro = _masked_ref(qf, kf, vf, masked, scale)
+        ro.backward(do.float())
+        with torch.no_grad():
+            s = qf.transpose(1, 2) @ kf.transpose(1, 2).repeat_interleave(Hq // Hkv, 1).mT * scale
+            rl = torch.logsumexp(s.masked_fill_(masked, float("-inf")), -1)
+            del s
+        assert torch.equal(torch.isfinite(lse), ~dead), (name, causal)
+        assert torch.allclose(lse[~dead], rl[~dead], rtol=1e-3, atol=2e-3), (name, causal)
+        assert (o.float() - ro).abs().max().item() < 3e-2, (name, causal)
+        assert dq.transpose(1, 2)[dead].float().abs().sum().item() == 0, (name, causal)
+        for nm, a, b in (("dq", dq, qf.grad), ("dk", dk, kf.grad), ("dv", dv, vf.grad)):
+            err = (a.float() - b).abs().max().item()
+            assert err <= 3e-2 * b.abs().max().item() + 2e-2, f"{name} {causal} {nm}: {err}"

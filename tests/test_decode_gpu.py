@@ -123,6 +123,43 @@ def test_skinny_gemm(M, K_, N, splits):
         assert (got.double() - ref).abs().le(ref.abs() * 2 ** -8 + 1e-4).all()
 
 
+@pytest.mark.parametrize("M,H,N", [(1, 512, 1536), (17, 2048, 5120), (128, 4096, 1024)])
+def test_skinny_gemm_behind_the_kernels_of_a_decode_step(M, H, N):
+    """As a decode step launches it, with weights fetched ahead of the wait: the norm kernel just before writes x and the residual,
+    another product just before writes x, and the same chain replayed from a CUDA graph."""
+    from paddle_b200.ops import native, _lib
+    torch.manual_seed(M)
+    h, r = torch.randn(M, H, device="cuda").bfloat16(), torch.randn(M, H, device="cuda").bfloat16()
+    ln = torch.randn(H, device="cuda").bfloat16()
+    w1, w2 = ((torch.randn(*s, device="cuda") * 0.05).bfloat16() for s in ((H, N), (N // 2, H)))
+
+    def step():
+        y, _, s = native.rms_norm_fwd(h, ln, 1e-5, residual=r, want_residual_out=True)
+        a = native.gemm_skinny(y, w1, swiglu=True, weights_ready=True)
+        return y, s, a, native.gemm_skinny(a, w2, residual=s, weights_ready=True)
+
+    def check(y, s, a, out):
+        assert torch.equal(s, (h.float() + r.float()).bfloat16())
+        g, u = (y.double() @ w1.double()).chunk(2, 1)
+        ref = torch.nn.functional.silu(g) * u
+        # one rounding to bf16; the fp32 sums and silu's exponential and quotient are good to 1e-6 of their terms
+        assert (a.double() - ref).abs().le(ref.abs() * 2 ** -8 + 1e-3).all()
+        ref = a.double() @ w2.double() + s.double()
+        assert (out.double() - ref).abs().le(ref.abs() * 2 ** -8 + 1e-3).all()
+    for _ in range(3):
+        check(*step())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = step()
+    for seed in (1, 2):
+        h.copy_(torch.randn(M, H, generator=torch.Generator().manual_seed(seed)))
+        w1.mul_(-1.0)                                   # weights written between two replays
+        graph.replay()
+        check(*outs)
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("M,Hq,Hkv,K_", [(1, 2, 2, 256), (5, 4, 1, 520), (33, 8, 2, 1024), (100, 4, 4, 512)])
 @pytest.mark.parametrize("with_bias", [False, True])
 def test_skinny_qkv_matches_separate_steps(M, Hq, Hkv, K_, with_bias):
