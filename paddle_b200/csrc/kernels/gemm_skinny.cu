@@ -13,8 +13,8 @@
 // [F, 2F); a tile takes 64 of each and stores silu(gate) * up: the [M, 2F] product never reaches memory), kQkv (a tile is one
 // head: bias, rotary embedding, q stored densely, k / v appended to their cache pages).
 //
-// Launched as a programmatic dependent: set-up, and with `weights_ready` the first 64 to 80 KB of weights per CTA, run under
-// the end of the kernel before.
+// Launched as a programmatic dependent: set-up, and with `weights_ready` the first weights of each CTA (a full ring: 80 KB up to
+// 16 rows, 64 KB up to 64, 48 KB above), run under the end of the kernel before.
 // Measured in a replayed decode step: gate / up of a 7B layer (180 MB) with its activation 30.2 us for one row (5.97 TB/s; before,
 // 256 x 256 tiles and a separate activation: 72 us); qkv, out and down projections of two layers 89 us (before, 128 x 256 tiles
 // with split-K atomics and a finalising kernel each: 123 us).  Two 7B layers and the head for one sequence, 1.07 GB of weights

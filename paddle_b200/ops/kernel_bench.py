@@ -205,16 +205,18 @@ def bench_decode(args, timer, hbm, tf):
         s = native.suggest_splits(M, N, K_)
         acc = torch.zeros(M, N, device="cuda", dtype=torch.float32)
 
-        def run():
+        def splitk():                                  # what batches above 128 rows take
             if s > 1:
                 native.gemm_splitk(x, w, acc, s)
                 native.splitk_finalize(acc)
             else:
-                native.gemm(x, w)
-        t = timer(run, args.iters)
+                native.gemm(x, w, max_ctas=1 << 30)    # the 256-row tiles
+        t = timer(lambda: native.gemm_skinny(x, w), args.iters)
+        t_one = timer(lambda: native.gemm_skinny(x[:1], w), args.iters)
+        t_split = timer(splitk, args.iters)
         by = 2.0 * K_ * N
-        rec = dict(op="skinny_gemm", name=name, M=M, N=N, K=K_, splits=s, ms=t, gbs=by / t / 1e6,
-                   frac_of_measured=by / t / 1e6 / hbm)
+        rec = dict(op="skinny_gemm", name=name, M=M, N=N, K=K_, ms=t, gbs=by / t / 1e6, frac_of_measured=by / t / 1e6 / hbm,
+                   one_row_ms=t_one, one_row_gbs=by / t_one / 1e6, splits=s, splitk_ms=t_split)
         if not args.no_baseline:
             t2 = timer(lambda: torch.matmul(x, w), args.iters)
             rec.update(lib_ms=t2, lib_gbs=by / t2 / 1e6)
