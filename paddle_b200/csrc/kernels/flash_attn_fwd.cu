@@ -396,7 +396,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // row's maximum, the more of the large probabilities are near 1, which bf16 holds exactly.  Relative error of O against
       // 64 bits with 64 / 128 keys: S=130 H=40 0.00224 / 0.00217, B=4 S=1024 H=40 causal 0.002055 / 0.002039, S=4096 H=32
       // causal 0.002111 / 0.002098; time 8.2 / 8.2, 65.6 / 67.6, 122.8 / 126.8 us.
-      ok = mbar_wait_warp(&bars->s_full[t][1], 0, abort_flag, p.status, 302 + t);
+      // Both buffers' first phases are observed here: a later wait for the second phase of one would pass over a first that is missing.
+      ok = mbar_wait_warp2(&bars->s_full[t][0], &bars->s_full[t][1], 0, abort_flag, p.status, 302 + t);
       if (ok) {
         tc_fence_after();
         uint32_t r0[BU / 32][32], r1[BU / 32][32];

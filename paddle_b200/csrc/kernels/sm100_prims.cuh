@@ -105,12 +105,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
   }
 }
-// A converged warp waits: every lane observes the phase itself, one look when it is complete already.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int site) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+// A converged warp waits until `look` holds for every lane: one look when it does already.
+template <typename Look>
+__device__ __forceinline__ bool wait_warp_until(Look look, uint32_t parity, volatile int* abort_flag, int* status, int site) {
+  if (__all_sync(0xffffffffu, look())) return true;
   unsigned long long t0 = 0;
 #pragma unroll 1
-  for (uint32_t i = 1; !__all_sync(0xffffffffu, mbar_try_wait(bar, parity)); ++i) {
+  for (uint32_t i = 1; !__all_sync(0xffffffffu, look()); ++i) {
     if ((i & 63u) != 0) continue;
     const unsigned long long now = globaltimer_ns();
     if (t0 == 0) t0 = now;
@@ -122,6 +123,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
     if (__any_sync(0xffffffffu, late || *abort_flag != 0)) return false;
   }
   return true;
+}
+// Every lane observes the phase itself.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int site) {
+  return wait_warp_until([&] { return mbar_try_wait(bar, parity); }, parity, abort_flag, status, site);
+}
+// The same phase of two barriers, both looked at together.
+__device__ __forceinline__ bool mbar_wait_warp2(uint64_t* a, uint64_t* b, uint32_t parity, volatile int* abort_flag, int* status, int site) {
+  return wait_warp_until([&] { return mbar_try_wait(a, parity) & mbar_try_wait(b, parity); }, parity, abort_flag, status, site);
 }
 // Same, but never raises the abort flag nor reports: used while draining after an abort.
 __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
