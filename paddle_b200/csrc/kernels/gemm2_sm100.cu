@@ -143,10 +143,17 @@ __device__ __forceinline__ void load_half(void* dst, const CUtensorMap* tm, uint
   }
 }
 
-template <bool A_MN, bool B_MN, int EPI, int TILE_N>
+constexpr int MAX_GROUPS = 8;
+// The operands of G products of the same M x N, worked on one after the other in one launch; K differs.
+template <int G>
+struct Operands {
+  CUtensorMap a[G], b[G], c[G];
+  int k[G];
+};
+
+template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
-gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int mn3d, int splits, int* status,
+gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int N, int mn3d, int splits, int* status,
                   const __nv_bfloat16* bias, int act) {
   constexpr int STAGES = stages(TILE_N), BN_HALF = TILE_N / 2, B_STAGE_BYTES = b_stage_bytes(TILE_N);
   constexpr uint32_t TM_COLS = 2 * TILE_N;
@@ -165,9 +172,15 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const bool leader = cta_rank == 0;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
   const int tiles_m = (M + TILE_M - 1) / TILE_M, tiles_n = (N + TILE_N - 1) / TILE_N;
-  const int KB_total = (K + BK - 1) / BK;
-  const int KBS = (KB_total + splits - 1) / splits;
-  const int num_tiles = tiles_m * tiles_n * splits;
+  const int group_tiles = tiles_m * tiles_n * splits;
+  const int num_tiles = group_tiles * (G == 1 ? 1 : groups);
+  // tile t: which product it belongs to, its number in that one, its blocks of K
+  auto group_of = [&](int t) { return G == 1 ? 0 : t / group_tiles; };
+  auto k_range = [&](int g, int t, int& kb0, int& kb1) {
+    const int kb_total = (op.k[g] + BK - 1) / BK, kbs = (kb_total + splits - 1) / splits;
+    kb0 = (t % splits) * kbs;
+    kb1 = min(kb_total, kb0 + kbs);
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -193,24 +206,25 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   if (warp == 4) {
     // ------------------------------------------------------------ TMA producer (one per CTA: its halves of A and B)
     if (lane == 0) {
-      prefetch_tmap(&tmA);
-      prefetch_tmap(&tmB);
+      prefetch_tmap(&op.a[0]);
+      prefetch_tmap(&op.b[0]);
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
       int issued = 0;
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters) {
-        int tm, tn;
-        tile_coords(t / splits, tiles_m, tiles_n, tm, tn);
+        int tm, tn, kb0, kb1;
+        const int g = group_of(t), tg = t - g * group_tiles;
+        tile_coords(tg / splits, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * TILE_M + static_cast<int>(cta_rank) * BM;
         const int n0 = tn * TILE_N + static_cast<int>(cta_rank) * BN_HALF;
-        const int kb0 = (t % splits) * KBS, kb1 = min(KB_total, kb0 + KBS);
+        k_range(g, tg, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&bars->empty[s], ph ^ 1, abort_flag, status, 100 + s)) { ok = false; break; }
           if (leader) mbar_expect_tx(&bars->full[s], 2 * (A_STAGE_BYTES + B_STAGE_BYTES));
           const int k0 = kb * BK;
-          load_half<A_MN, BM>(sA + s * A_STAGE_BYTES, &tmA, &bars->full[s], m0, k0, (mn3d & 1) != 0);
-          load_half<B_MN, BN_HALF>(sB + s * B_STAGE_BYTES, &tmB, &bars->full[s], n0, k0, (mn3d & 2) != 0);
+          load_half<A_MN, BM>(sA + s * A_STAGE_BYTES, &op.a[g], &bars->full[s], m0, k0, (mn3d & 1) != 0);
+          load_half<B_MN, BN_HALF>(sB + s * B_STAGE_BYTES, &op.b[g], &bars->full[s], n0, k0, (mn3d & 2) != 0);
           ++issued;
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
@@ -241,7 +255,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (!mbar_wait_warp(&bars->tempty[acc], acc_ph ^ 1, abort_flag, status, 200 + acc)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tm + acc * TILE_N;
-        const int kb0 = (t % splits) * KBS, kb1 = min(KB_total, kb0 + KBS);
+        const int g = group_of(t);
+        int kb0, kb1;
+        k_range(g, t - g * group_tiles, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_warp(&bars->full[s], ph, abort_flag, status, 300 + s)) { ok = false; break; }
           tc_fence_after();
@@ -273,7 +289,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     int chunk_counter = 0;
     for (int t = cluster_id; t < num_tiles; t += n_clusters, ++it) {
       int tm, tn;
-      tile_coords(t / splits, tiles_m, tiles_n, tm, tn);
+      const int g = group_of(t);
+      tile_coords((t - g * group_tiles) / splits, tiles_m, tiles_n, tm, tn);
       const int m0 = tm * TILE_M + static_cast<int>(cta_rank) * BM, n0 = tn * TILE_N;
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
@@ -375,9 +392,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             else mbar_arrive_remote(&bars->tempty[acc], 0);
           }
           if (rows_live && n0 + c * CW < N) {
-            if (EPI == kAccumF32) tma_reduce_add_2d(&tmC, stage, n0 + c * CW, m0);
-            else if (EPI == kSwiglu) tma_store_2d(&tmC, stage, (n0 + c * CW) / 2, m0);
-            else tma_store_2d(&tmC, stage, n0 + c * CW, m0);
+            if (EPI == kAccumF32) tma_reduce_add_2d(&op.c[g], stage, n0 + c * CW, m0);
+            else if (EPI == kSwiglu) tma_store_2d(&op.c[g], stage, (n0 + c * CW) / 2, m0);
+            else tma_store_2d(&op.c[g], stage, n0 + c * CW, m0);
           }
           tma_commit_group();
         }
@@ -399,20 +416,19 @@ static int max_clusters(int max_ctas) {
   return clusters < 1 ? 1 : clusters;
 }
 
-template <bool A_MN, bool B_MN, int EPI, int TILE_N>
-static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, int M, int N, int K,
-                          int mn3d, int* status, cudaStream_t stream, int max_ctas, int splits,
-                          const __nv_bfloat16* bias = nullptr, int act = 0) {
-  auto kfn = gemm2_bf16_kernel<A_MN, B_MN, EPI, TILE_N>;
+template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G = 1>
+static int launch_variant(const Operands<G>& op, int groups, int M, int N, int mn3d, int* status, cudaStream_t stream, int max_ctas,
+                          int splits, const __nv_bfloat16* bias = nullptr, int act = 0) {
+  auto kfn = gemm2_bf16_kernel<A_MN, B_MN, EPI, TILE_N, G>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(TILE_N)) != cudaSuccess) return kErrCuda;
     configured = true;
   }
-  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N) * splits;
+  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N) * splits * groups;
   int clusters = max_clusters(max_ctas);
   if (clusters > tiles) clusters = tiles;
-  kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(tmA, tmB, tmC, M, N, K, mn3d, splits, status, bias, act);
+  kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(op, groups, M, N, mn3d, splits, status, bias, act);
   return cudaGetLastError() == cudaSuccess ? kLaunchOk : kErrCuda;
 }
 
@@ -447,20 +463,21 @@ PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, in
   if (!aligned16(A) || !aligned16(B) || !aligned16(C)) return kErrAlignment;
   if ((lda % 8) || (ldb % 8) || (epi == kStoreBf16 ? (ldc % 8) : (ldc % 4))) return kErrAlignment;
   const int TN = tile_n(M, N, splits, max_ctas), BN_HALF = TN / 2;
-  CUtensorMap tmA, tmB, tmC;
+  Operands<1> op;
+  op.k[0] = K;
   bool ok = true;
   int a3d = 0, b3d = 0;
-  if (!a_mn_major) ok &= encode_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, A, K, M, uint64_t(lda) * 2, BK, BM);
-  else ok &= encode_tmap_mn(&tmA, A, M, K, uint64_t(lda) * 2, BM / 64, BK, &a3d);
-  if (!b_mn_major) ok &= encode_tmap_2d(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, B, K, N, uint64_t(ldb) * 2, BK, BN_HALF);
-  else ok &= encode_tmap_mn(&tmB, B, N, K, uint64_t(ldb) * 2, BN_HALF / 64, BK, &b3d);
-  if (epi == kStoreBf16) ok &= encode_tmap_2d(&tmC, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, C, N, M, uint64_t(ldc) * 2, 64, BM);
-  else ok &= encode_tmap_2d(&tmC, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, C, N, M, uint64_t(ldc) * 4, 32, BM);
+  if (!a_mn_major) ok &= encode_tmap_2d(&op.a[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, A, K, M, uint64_t(lda) * 2, BK, BM);
+  else ok &= encode_tmap_mn(&op.a[0], A, M, K, uint64_t(lda) * 2, BM / 64, BK, &a3d);
+  if (!b_mn_major) ok &= encode_tmap_2d(&op.b[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, B, K, N, uint64_t(ldb) * 2, BK, BN_HALF);
+  else ok &= encode_tmap_mn(&op.b[0], B, N, K, uint64_t(ldb) * 2, BN_HALF / 64, BK, &b3d);
+  if (epi == kStoreBf16) ok &= encode_tmap_2d(&op.c[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, C, N, M, uint64_t(ldc) * 2, 64, BM);
+  else ok &= encode_tmap_2d(&op.c[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, C, N, M, uint64_t(ldc) * 4, 32, BM);
   if (!ok) return kErrTensorMap;
 #define PD_GEMM2_CASE(AM, BM_, E)                                                                  \
   if (a_mn_major == AM && b_mn_major == BM_ && epi == E)                                           \
-    return TN == 128 ? launch_variant<AM, BM_, E, 128>(tmA, tmB, tmC, M, N, K, a3d | (b3d << 1), status, stream, max_ctas, splits) \
-                     : launch_variant<AM, BM_, E, 256>(tmA, tmB, tmC, M, N, K, a3d | (b3d << 1), status, stream, max_ctas, splits);
+    return TN == 128 ? launch_variant<AM, BM_, E, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, max_ctas, splits) \
+                     : launch_variant<AM, BM_, E, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, max_ctas, splits);
   PD_GEMM2_CASE(0, 0, 0) PD_GEMM2_CASE(0, 1, 0) PD_GEMM2_CASE(1, 0, 0) PD_GEMM2_CASE(1, 1, 0)
   PD_GEMM2_CASE(0, 0, 1) PD_GEMM2_CASE(0, 1, 1) PD_GEMM2_CASE(1, 0, 1) PD_GEMM2_CASE(1, 1, 1)
   PD_GEMM2_CASE(0, 0, 2) PD_GEMM2_CASE(0, 1, 2) PD_GEMM2_CASE(1, 0, 2) PD_GEMM2_CASE(1, 1, 2)
@@ -480,23 +497,80 @@ PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M
   if (!aligned16(A) || !aligned16(B) || !aligned16(C)) return kErrAlignment;
   if ((lda % 8) || (ldb % 8) || (ldc % 8)) return kErrAlignment;
   const int TN = swiglu ? 256 : tile_n(M, N, 1, 0), BN_HALF = TN / 2;
-  CUtensorMap tmA, tmB, tmC;
+  Operands<1> op;
+  op.k[0] = K;
   bool ok = true;
   int a3d = 0, b3d = 0;
-  if (!a_mn_major) ok &= encode_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, A, K, M, uint64_t(lda) * 2, BK, BM);
-  else ok &= encode_tmap_mn(&tmA, A, M, K, uint64_t(lda) * 2, BM / 64, BK, &a3d);
-  if (!b_mn_major) ok &= encode_tmap_2d(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, B, K, N, uint64_t(ldb) * 2, BK, BN_HALF);
-  else ok &= encode_tmap_mn(&tmB, B, N, K, uint64_t(ldb) * 2, BN_HALF / 64, BK, &b3d);
-  ok &= encode_tmap_2d(&tmC, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, C, swiglu ? N / 2 : N, M, uint64_t(ldc) * 2, 64, BM);
+  if (!a_mn_major) ok &= encode_tmap_2d(&op.a[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, A, K, M, uint64_t(lda) * 2, BK, BM);
+  else ok &= encode_tmap_mn(&op.a[0], A, M, K, uint64_t(lda) * 2, BM / 64, BK, &a3d);
+  if (!b_mn_major) ok &= encode_tmap_2d(&op.b[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, B, K, N, uint64_t(ldb) * 2, BK, BN_HALF);
+  else ok &= encode_tmap_mn(&op.b[0], B, N, K, uint64_t(ldb) * 2, BN_HALF / 64, BK, &b3d);
+  ok &= encode_tmap_2d(&op.c[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, C, swiglu ? N / 2 : N, M, uint64_t(ldc) * 2, 64, BM);
   if (!ok) return kErrTensorMap;
   const __nv_bfloat16* bp = static_cast<const __nv_bfloat16*>(bias);
 #define PD_GEMM2_EPI_CASE(AM, BM_)                                                                              \
   if (a_mn_major == AM && b_mn_major == BM_) {                                                                  \
-    if (swiglu) return launch_variant<AM, BM_, kSwiglu, 256>(tmA, tmB, tmC, M, N, K, a3d | (b3d << 1), status, stream, 0, 1); \
-    return TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(tmA, tmB, tmC, M, N, K, a3d | (b3d << 1), status, stream, 0, 1, bp, act) \
-                     : launch_variant<AM, BM_, kBiasAct, 256>(tmA, tmB, tmC, M, N, K, a3d | (b3d << 1), status, stream, 0, 1, bp, act); \
+    if (swiglu) return launch_variant<AM, BM_, kSwiglu, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1); \
+    return TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act) \
+                     : launch_variant<AM, BM_, kBiasAct, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act); \
   }
   PD_GEMM2_EPI_CASE(0, 0) PD_GEMM2_EPI_CASE(0, 1) PD_GEMM2_EPI_CASE(1, 0) PD_GEMM2_EPI_CASE(1, 1)
 #undef PD_GEMM2_EPI_CASE
   return kErrBadShape;
+}
+
+// Weight gradients of several experts:  C_g[M, N] (=|+=) A_g^T B_g for the rows [starts[g], starts[g] + rows[g]) of A [*, M] and
+// B [*, N] (bf16).  C: fp32, added into (accumulate = 1), or bf16, `c_stride` elements apart; starts / rows: host arrays.  A product
+// without rows is left out.  One launch takes up to MAX_GROUPS products, the longest first: a launch each pays its own ramp and last
+// wave (us, launches each -> one; 8192 rows of 4 experts, 4096 x 8192 into fp32 438 -> 425, 4096 x 4096 241 -> 204; of 8 experts
+// 4096 x 7168 568 -> 489; 4096 rows of 8, 2048 x 3584 169 -> 119; 256 rows of 8, 512 x 512 54 -> 9).
+PD_EXPORT int pd_gemm_bf16_grouped_tn(const void* A, const void* B, void* C, const int64_t* starts, const int64_t* rows, int groups,
+                                      int M, int N, int lda, int ldb, int ldc, int64_t c_stride, int accumulate, int* status,
+                                      cudaStream_t stream) {
+  using namespace pd;
+  using namespace pd::gemm2;
+  if (M <= 0 || N <= 0 || groups < 0) return kErrBadShape;
+  if (!aligned16(A) || !aligned16(B) || !aligned16(C)) return kErrAlignment;
+  if ((lda % 8) || (ldb % 8) || (accumulate ? (ldc % 4) || (c_stride % 4) : (ldc % 8) || (c_stride % 8))) return kErrAlignment;
+  const int elem = accumulate ? 4 : 2;
+  int left = 0;
+  for (int g = 0; g < groups; ++g) {
+    if (rows[g] < 0 || rows[g] > INT32_MAX) return kErrBadShape;
+    left += rows[g] > 0;
+  }
+  Operands<MAX_GROUPS> op;
+  int64_t below_rows = INT64_MAX;      // of the product taken last; equal ones are taken in their order
+  int below_g = -1;
+  while (left > 0) {
+    const int n = left < MAX_GROUPS ? left : MAX_GROUPS, TN = tile_n(M, N, n, 0);
+    int a3d = 0, b3d = 0;
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+      int best = -1;
+      for (int g = 0; g < groups; ++g) {
+        const bool open = rows[g] > 0 && (rows[g] < below_rows || (rows[g] == below_rows && g > below_g));
+        if (open && (best < 0 || rows[g] > rows[best])) best = g;
+      }
+      below_rows = rows[best];
+      below_g = best;
+      op.k[i] = static_cast<int>(rows[best]);
+      ok &= encode_tmap_mn(&op.a[i], static_cast<const __nv_bfloat16*>(A) + starts[best] * lda, M, rows[best], uint64_t(lda) * 2, BM / 64, BK, &a3d);
+      ok &= encode_tmap_mn(&op.b[i], static_cast<const __nv_bfloat16*>(B) + starts[best] * ldb, N, rows[best], uint64_t(ldb) * 2, TN / 2 / 64, BK, &b3d);
+      ok &= encode_tmap_2d(&op.c[i], accumulate ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                           static_cast<char*>(C) + best * c_stride * elem, N, M, uint64_t(ldc) * elem, accumulate ? 32 : 64, BM);
+    }
+    if (!ok) return kErrTensorMap;
+    for (int i = n; i < MAX_GROUPS; ++i) op.a[i] = op.a[0], op.b[i] = op.b[0], op.c[i] = op.c[0], op.k[i] = 0;
+    const int mn3d = a3d | (b3d << 1);
+    int rc;
+    if (accumulate)
+      rc = TN == 128 ? launch_variant<true, true, kAccumF32, 128, MAX_GROUPS>(op, n, M, N, mn3d, status, stream, 0, 1)
+                     : launch_variant<true, true, kAccumF32, 256, MAX_GROUPS>(op, n, M, N, mn3d, status, stream, 0, 1);
+    else
+      rc = TN == 128 ? launch_variant<true, true, kStoreBf16, 128, MAX_GROUPS>(op, n, M, N, mn3d, status, stream, 0, 1)
+                     : launch_variant<true, true, kStoreBf16, 256, MAX_GROUPS>(op, n, M, N, mn3d, status, stream, 0, 1);
+    if (rc != kLaunchOk) return rc;
+    left -= n;
+  }
+  return kLaunchOk;
 }

@@ -7,8 +7,8 @@ stacked (``[E, K, N]``) and all experts run in one launch per GEMM:
 
 * forward   ``Y = grouped(Xq, Wq)``          X quantised per 1 x 128 block, W per 128 x 128 block (e4m3, fp32 scales)
 * dgrad     ``dX = grouped(dYq, (W^T)q)``    the same kernel on a byte-transposed copy of the e4m3 weights
-* wgrad     ``dW[e] = X_e^T dY_e``           bf16 operands on the plain tcgen05 GEMM, fp32 accumulation into
-                                            ``main_grad`` when the parameter carries one
+* wgrad     ``dW[e] = X_e^T dY_e``           bf16 operands on the plain tcgen05 GEMM, all experts in one launch, fp32
+                                            accumulation into ``main_grad`` when the parameter carries one
 
 Quantised weights are cached between optimizer steps (micro-batches of one step reuse them) and keyed on the
 parameter's version counter, which this library's optimizers advance; ``weights_updated()`` drops them by hand for
@@ -82,17 +82,11 @@ class _GroupedLinearFP8(torch.autograd.Function):
             dx = native.grouped_gemm_fp8(dq, ds, wq, ws, offsets)
         if ctx.needs_input_grad[1]:
             mg = getattr(ctx.w_ref, "main_grad", None)
-            if mg is None:
+            if mg is not None:
+                native.gemm_grouped_tn(x, dy, ctx.counts, mg, accumulate=True)
+            else:
                 dw = torch.zeros_like(w)
-            start = 0
-            for e, n in enumerate(ctx.counts):
-                if n:
-                    xe, de = x[start:start + n], dy[start:start + n]
-                    if mg is not None:
-                        native.gemm(xe, de, trans_a=True, out=mg[e], accumulate=True)
-                    else:
-                        native.gemm(xe, de, trans_a=True, out=dw[e])
-                start += n
+                native.gemm_grouped_tn(x, dy, ctx.counts, dw)
         return dx, dw, None, None, None
 
 

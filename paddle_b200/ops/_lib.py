@@ -55,7 +55,7 @@ def _load(name: str, builder: str):
 # wraps each in a ctypes object.
 _SIGNATURES = {
     "pd_gemm_bf16_2cta": "ppp iiiiiiiiiii pp", "pd_gemm_bf16_2cta_epi": "ppp iiiiiiii p ii pp",
-    "pd_gemm_skinny": "ppp iiiiii pp iiii pp",
+    "pd_gemm_skinny": "ppp iiiiii pp iiii pp", "pd_gemm_bf16_grouped_tn": "ppppp iiiiii l i pp",
     "pd_rms_norm_fwd": "ppp i ppp l i f p", "pd_rms_norm_bwd": "ppp i ppppp i l i p", "pd_rms_norm_bwd_parts": "l",
     "pd_rope": "ppppp l ii ll iii p", "pd_swiglu_fwd": "ppp l i l p", "pd_swiglu_bwd": "ppppp l i l p",
     "pd_ce_stats": "p i ppppp l i ll p", "pd_ce_bwd": "p i ppp i p l i ll f p",

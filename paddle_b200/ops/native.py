@@ -107,6 +107,36 @@ def gemm(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: bool 
     return out
 
 
+@plain_dispatch
+def gemm_grouped_tn(a: torch.Tensor, b: torch.Tensor, counts, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
+    """``out[g] (=|+=) a_g^T @ b_g`` for consecutive groups of ``counts[g]`` rows of ``a`` [rows, M] and ``b`` [rows, N]: the weight
+    gradients of several experts.  ``accumulate=True`` adds into an fp32 ``out`` [G, M, N], otherwise a bf16 one is written; a group
+    without rows leaves its matrix as it is."""
+    _req(a.dtype == BF16 and b.dtype == BF16 and a.dim() == 2 and b.dim() == 2, "gemm_grouped_tn: 2-D bf16 operands required")
+    _req(a.stride(1) == 1 and b.stride(1) == 1, "gemm_grouped_tn: operands need a unit inner stride")
+    G, M, N = len(counts), a.shape[1], b.shape[1]
+    _req(tuple(out.shape) == (G, M, N) and out.stride(2) == 1, "gemm_grouped_tn: bad `out`")
+    _req(out.dtype == (F32 if accumulate else BF16), "gemm_grouped_tn: `out` is fp32 when it is added into, bf16 otherwise")
+    rows = min(a.shape[0], b.shape[0])
+    starts, ns, at = [], [], 0
+    for n in counts:                             # rows past the last one do not exist: a slice would end there as well
+        _req(n >= 0, "gemm_grouped_tn: negative count")
+        starts.append(min(at, rows))
+        ns.append(min(at + n, rows) - starts[-1])
+        at += n
+    if GEMM_IMPL != "2cta":
+        for g, (s, n) in enumerate(zip(starts, ns)):
+            if n:
+                gemm(a[s:s + n], b[s:s + n], trans_a=True, out=out[g], accumulate=accumulate)
+        return out
+    rc = _lib.kernels().pd_gemm_bf16_grouped_tn(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), (c_int64 * G)(*starts), (c_int64 * G)(*ns), G, M, N, a.stride(0), b.stride(0),
+        out.stride(1), out.stride(0), 1 if accumulate else 0, _lib.status_buffer(a.device).data_ptr(), raw_stream())
+    check(rc, "pd_gemm_bf16_grouped_tn")
+    _count((sum(1 for n in ns if n) + 7) // 8)
+    return out
+
+
 # --------------------------------------------------------------------------------------------- norms
 @plain_dispatch
 def rms_norm_fwd(x, w, eps, residual=None, want_residual_out=False):

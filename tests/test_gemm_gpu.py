@@ -150,3 +150,28 @@ def test_tile_width_follows_the_ctas_a_call_may_use(max_ctas):
     torch.cuda.synchronize()
     _lib.check_status()
     assert (got.double() - ref).abs().le(ref.abs() * 2 ** -8 + 1e-3).all()      # fp32 sums of products of size 1, one rounding
+
+
+@pytest.mark.parametrize("M,N,counts", [(136, 144, [70, 0, 1, 64, 65]), (512, 264, [300, 129, 300]), (1024, 2048, [128] * 9 + [0, 500]), (256, 256, [0, 0])])
+def test_gemm_grouped_weight_gradients(M, N, counts):
+    """Uneven, equal, empty and more groups than one launch takes, on ragged sizes; rows past the counted ones are not read."""
+    from paddle_b200.ops import _lib, native
+    rows = sum(counts)
+    a, b = _mk(M, N, max(rows, 1) + 40, True, False)
+    a[rows:], b[rows:] = float("nan"), float("nan")
+    acc = torch.randn(len(counts), M, N, device="cuda")
+    start, plain = acc.clone(), torch.full((len(counts), M, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    native.gemm_grouped_tn(a, b, counts, acc, accumulate=True)
+    native.gemm_grouped_tn(a, b, counts, plain)
+    _lib.check_status()
+    s = 0
+    for g, n in enumerate(counts):
+        ref = _ref(a[s:s + n], b[s:s + n], True, False)
+        s += n
+        # products of bf16 are exact in fp32, n of them are summed: errors of n * 2^-24 relative to the sum of magnitudes (< 6 n)
+        tol = 6 * max(n, 1) * n * 2 ** -24 + 1e-5
+        assert (acc[g] - start[g] - ref).abs().max() <= tol + 2 ** -22 * (start[g].abs().max() + ref.abs().max())
+        if n:
+            assert ((plain[g].float() - ref).abs() <= 2 ** -8 * ref.abs() + tol).all()
+        else:
+            assert torch.equal(plain[g], torch.full_like(plain[g], 7.0))
