@@ -32,6 +32,11 @@
 // to 200 cycles each beside the MMAs, so all three barriers of a sub-tile are looked at together and dP^T is read with S^T; a warp of
 // its own stages the statistics, where a store and a 256-thread barrier stood in front of every sub-tile (438 -> 395 us causal);
 // MMAs issued from a one-lane branch and waits of three steps came before that.  (1) and (2) issued by a warp of their own: 2 % slower.
+// Long calls run at the power cap (990 W, 1600 MHz), where shared-memory traffic costs as much as cycles: sub-tiles of 128 queries, which
+// run every MMA at its full rate but read dS^T from shared memory for (4), took 416 / 734 us (causal / full) against 397 / 702.
+// The dQ accumulator is [B, Hq, Sq, 128], so the 64 additions of a thread share one address; it is cleared by the kernel that makes
+// Delta, and the conversion is launched ahead of this kernel's end: forward and backward of B=2 S=1999 H=32/8 599 -> 591 us, of B=1
+// S=4096 H=32 causal 625 -> 619 (the layout alone 397 -> 394 and 221 -> 218 for the backward call).
 #include <math.h>
 
 #include "host_utils.h"
@@ -67,7 +72,7 @@ struct Params {
   float scale, scale_log2;
   const float* lse;     // [B, Hq, Sq] natural log
   const float* delta;   // [B, Hq, Sq]
-  float* dq_acc;        // [B, Sq, Hq, 128], added into
+  float* dq_acc;        // [B, Hq, Sq, 128], added into
   int parts;            // CTAs that share the query heads of a group; with more than one each writes its own fp32 sums
   float* dkv_part;      // [parts, 2, B, Sk, Hkv, 128]: dK and dV of each part
   int* status;
@@ -137,6 +142,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int n_it = per_head * group;
 
   if (threadIdx.x == 0) {
+    pdl_trigger();                                   // the conversion of dQ: waits for this kernel before it reads anything
     mbar_init(&bars->kv_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&bars->qdo_full[s], 1);
@@ -482,7 +488,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // same rate: the L2 takes the 32 KB of a sub-tile from every SM in 0.8 us either way.
     const int dr = threadIdx.x - 128;                 // 0..127 = head-dim index = TMEM lane
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const size_t row_stride = static_cast<size_t>(p.Hq) * D;
+    constexpr int row_stride = D;                     // rows of a head lie one behind the other: all additions share one address
     int qh = qh0, tq = 0;
 #pragma unroll 1
     for (int it = 0; it < n_it; ++it) {
@@ -495,7 +501,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_before();
       mbar_arrive_warp(&bars->dq_empty[it & 1]);
       const int q0 = (t0 + tq) * BQ;
-      float* dst = p.dq_acc + (static_cast<size_t>(batch) * p.Sq + q0) * row_stride + static_cast<size_t>(qh) * D + dr;
+      float* dst = p.dq_acc + ((static_cast<size_t>(batch) * p.Hq + qh) * p.Sq + q0) * D + dr;
       const int live = p.Sq - q0;                     // rows of this sub-tile inside the matrix
       if (live >= BQ) {
 #pragma unroll
@@ -517,11 +523,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
-// delta[b, h, s] = sum_d dO * O: 16 lanes of 16 bytes per row, so two rows per warp, and four such pairs in flight (with one
+// delta[b, h, s] = sum_d dO * O, and the row of the dQ accumulator is cleared: 16 lanes of 16 bytes per row, so two rows per warp, and four such pairs in flight (with one
 // row of 8-byte loads per warp the 67 MB of S = 4096, H = 32 took 26 us)
 constexpr int DELTA_ROWS = 4;
 __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                                    float* __restrict__ delta, int64_t rows, int S, int H, int64_t o_tok,
+                                                    float* __restrict__ delta, float* __restrict__ dq_acc, int64_t rows, int S, int H, int64_t o_tok,
                                                     int64_t o_batch, int64_t do_tok, int64_t do_batch) {
   const int64_t first = (static_cast<int64_t>(blockIdx.x) * 16 + (threadIdx.x >> 4)) * DELTA_ROWS;
   const int c = (threadIdx.x & 15) * 8;
@@ -540,6 +546,13 @@ __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restr
   }
 #pragma unroll
   for (int k = 0; k < DELTA_ROWS; ++k) {
+    if (first + k < rows) {
+      float4* z = reinterpret_cast<float4*>(dq_acc + at[k] * D) + (threadIdx.x & 15);
+      z[0] = z[16] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < DELTA_ROWS; ++k) {
     const uint32_t u[4] = {a[k].x, a[k].y, a[k].z, a[k].w}, v[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
     float acc = 0.f;
 #pragma unroll
@@ -553,9 +566,10 @@ __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restr
   }
 }
 
-// dq (bf16, [B, S, H, 128] with token / batch strides) = dq_acc (fp32, contiguous); 16 threads of 8 values per row
+// dq (bf16, [B, S, H, 128] with token / batch strides) = dq_acc (fp32 [B, H, S, 128]); 16 threads of 8 values per row
 __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int64_t rows,
                                                          int S, int H, int64_t tok, int64_t batch) {
+  pdl_wait();
   const int64_t first = (static_cast<int64_t>(blockIdx.x) * 16 + (threadIdx.x >> 4)) * 2;
   const int c = (threadIdx.x & 15) * 8;
   float4 v[2][2];
@@ -569,10 +583,9 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict
   for (int k = 0; k < 2; ++k) {
     const int64_t row = first + k;
     if (row >= rows) break;
-    const int64_t bs = row / H;
-    const int h = static_cast<int>(row - bs * H);
-    const int64_t b = bs / S;
-    const int64_t s = bs - b * S;
+    const int64_t bh = row / S, s = row - bh * S;
+    const int64_t b = bh / H;
+    const int h = static_cast<int>(bh - b * H);
     *reinterpret_cast<uint4*>(dst + b * batch + s * tok + static_cast<int64_t>(h) * D + c) =
         make_uint4(pack_bf16x2(v[k][0].x, v[k][0].y), pack_bf16x2(v[k][0].z, v[k][0].w), pack_bf16x2(v[k][1].x, v[k][1].y),
                    pack_bf16x2(v[k][1].z, v[k][1].w));
@@ -641,7 +654,7 @@ PD_EXPORT int pd_flash_attn_bwd_parts(int B, int Sq, int Sk, int Hq, int Hkv, in
 }
 
 // dkv_part: null, or fp32 scratch [parts, 2, B, Sk, Hkv, 128] for `parts` (a divisor of Hq / Hkv) > 1 CTAs per key tile.
-// dq_acc: zero-initialised fp32 [B, Sq, Hq, 128] (contiguous); delta: fp32 [B, Hq, Sq] scratch;
+// dq_acc: fp32 scratch [B, Hq, Sq, 128], 16-byte aligned; delta: fp32 [B, Hq, Sq] scratch;
 // dq/dk/dv: bf16 outputs [B, S, H, 128] with their own token / batch strides (e.g. views of a packed dqkv).  
 PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, const void* v, const void* o,
                                 const float* lse, float* delta, float* dq_acc, float* dkv_part, void* dq, void* dk,
@@ -655,7 +668,7 @@ PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, c
   using namespace pd::fab;
   if (B <= 0 || Sq <= 0 || Sk <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0) return kErrBadShape;
   if (parts < 1 || (Hq / Hkv) % parts != 0 || (parts > 1 && dkv_part == nullptr)) return kErrBadShape;
-  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(d_o) || !aligned16(dkv_part)) return kErrAlignment;
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(d_o) || !aligned16(dkv_part) || !aligned16(dq_acc)) return kErrAlignment;
   if ((q_tok % 8) || (k_tok % 8) || (v_tok % 8) || (o_tok % 8) || (do_tok % 8)) return kErrAlignment;
   CUtensorMap tmQ, tmDO, tmK, tmV, tmDK, tmDV;
   bool ok = make_map_bf16(&tmQ, q, B, Sq, Hq, q_tok, q_batch, BQ) &&
@@ -674,7 +687,7 @@ PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, c
   }
   const int64_t rows = static_cast<int64_t>(B) * Sq * Hq;
   delta_kernel<<<static_cast<unsigned>((rows + 16 * DELTA_ROWS - 1) / (16 * DELTA_ROWS)), 256, 0, stream>>>(
-      (const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, rows, Sq, Hq, o_tok, o_batch, do_tok, do_batch);
+      (const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, dq_acc, rows, Sq, Hq, o_tok, o_batch, do_tok, do_batch);
   if (bounds != nullptr && (mask_heads != 1 && mask_heads != Hq && mask_heads != Hkv)) return kErrBadShape;
   if (bounds != nullptr && (!aligned16(bounds) || tile_bounds == nullptr || !aligned16(tile_bounds))) return kErrAlignment;
   Params p{B, Sq, Sk, Hq, Hkv, causal, scale, scale * 1.4426950408889634f, lse, delta, dq_acc, parts, dkv_part, status,
@@ -692,8 +705,10 @@ PD_EXPORT int pd_flash_attn_bwd(const void* d_o, const void* q, const void* k, c
   const unsigned grid = static_cast<unsigned>(grid64);
   if (bounds != nullptr) flash_bwd_kernel<true><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmQ, tmDO, tmK, tmV, tmDK, tmDV, p, static_cast<int>(chunk));
   else flash_bwd_kernel<false><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmQ, tmDO, tmK, tmV, tmDK, tmDV, p, static_cast<int>(chunk));
-  dq_convert_kernel<<<static_cast<unsigned>((rows + 31) / 32), 256, 0, stream>>>(dq_acc, (__nv_bfloat16*)dq, rows, Sq, Hq, dq_tok,
-                                                                                 dq_batch);
+  if (cudaGetLastError() != cudaSuccess) return kErrCuda;
+  const int rc = launch_pdl(dq_convert_kernel, dim3(static_cast<unsigned>((rows + 31) / 32)), dim3(256), 0, stream, 1, dq_acc,
+                            (__nv_bfloat16*)dq, rows, Sq, Hq, dq_tok, dq_batch);
+  if (rc != kLaunchOk) return rc;
   if (parts > 1) {
     const int64_t kv_rows = static_cast<int64_t>(B) * Sk * Hkv;
     dkv_convert_kernel<<<dim3(static_cast<unsigned>((kv_rows + 15) / 16), 2), 256, 0, stream>>>(

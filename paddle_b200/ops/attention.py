@@ -82,14 +82,16 @@ def bwd(do, q, k, v, o, lse, causal, scale, dq=None, dk=None, dv=None, mask=None
     dk = torch.empty((B, Sk, Hkv, D), dtype=torch.bfloat16, device=dev) if dk is None else dk
     dv = torch.empty((B, Sk, Hkv, D), dtype=torch.bfloat16, device=dev) if dv is None else dv
     assert _view_ok(dq) and _view_ok(dk) and _view_ok(dv)
-    # fp32 accumulator of dq, and the sums of dk / dv of each CTA when several share a key tile (few kv heads)
+    # scratch: the fp32 accumulator of dq, the sums of dk / dv of each CTA when several share a key tile (few kv heads), delta
     parts = _lib.kernels().pd_flash_attn_bwd_parts(B, Sq, Sk, Hq, Hkv, 1 if causal else 0)
-    dq_acc = torch.zeros(B * Sq * Hq * D, dtype=torch.float32, device=dev)
-    dkv_part = torch.empty(parts * 2 * B * Sk * Hkv * D, dtype=torch.float32, device=dev) if parts > 1 else None
-    delta = torch.empty((B, Hq, Sq), dtype=torch.float32, device=dev)
+    rows = B * Sq * Hq
+    n_part = parts * 2 * B * Sk * Hkv * D if parts > 1 else 0
+    scratch = torch.empty(rows * D + n_part + rows, dtype=torch.float32, device=dev)
+    dq_acc = scratch.data_ptr()
+    dkv_part = dq_acc + 4 * rows * D
     rc = _lib.kernels().pd_flash_attn_bwd(
-        addr(do), addr(q), addr(k), addr(v), addr(o), addr(lse), addr(delta), addr(dq_acc),
-        addr(dkv_part), addr(dq), addr(dk),
+        addr(do), addr(q), addr(k), addr(v), addr(o), addr(lse), dkv_part + 4 * n_part, dq_acc,
+        dkv_part if n_part else 0, addr(dq), addr(dk),
         addr(dv), B, Sq, Sk, Hq, Hkv,
         q.stride(1), q.stride(0), k.stride(1), k.stride(0),
         v.stride(1), v.stride(0), o.stride(1), o.stride(0),
