@@ -36,7 +36,7 @@ constexpr int smem_bytes(int tn) { return stages(tn) * (A_STAGE_BYTES + b_stage_
 constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;   // clears the CTA-pair bit of a shared::cluster address -> leader CTA
 
 enum Epi : int { kStoreBf16 = 0, kStoreF32 = 1, kAccumF32 = 2, kBiasAct = 3, kSwiglu = 4 };
-// kBiasAct: C = act(A B + bias) as bf16 (bias bf16 [N] or null; act: 0 none, 1 relu, 2 gelu (erf), 3 gelu (tanh),
+// kBiasAct: C = act(A B + bias) + residual as bf16 (bias bf16 [N], residual bf16 [M, N], each or null; act: 0 none, 1 relu, 2 gelu (erf), 3 gelu (tanh),
 // 4 silu) - the reference's fused_gemm_epilogue (paddle/phi/kernels/fusion/gpu/fused_gemm_epilogue_kernel.cu).
 // kSwiglu: the N columns hold (gate, up) pairs interleaved; C [M, N / 2] = silu(gate) * up as bf16, i.e. the first
 // feed-forward GEMM with its activation, without the [M, N] intermediate ever reaching memory.
@@ -154,7 +154,7 @@ struct Operands {
 template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int N, int mn3d, int splits, int* status,
-                  const __nv_bfloat16* bias, int act) {
+                  const __nv_bfloat16* bias, int act, const __nv_bfloat16* residual, int ldr) {
   constexpr int STAGES = stages(TILE_N), BN_HALF = TILE_N / 2, B_STAGE_BYTES = b_stage_bytes(TILE_N);
   constexpr uint32_t TM_COLS = 2 * TILE_N;
   extern __shared__ uint8_t smem_raw[];
@@ -362,6 +362,23 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
 #pragma unroll
                 for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(apply_act(__uint_as_float(r[i]), act));
               }
+              // a residual added by a kernel of its own moves the product through memory twice more: a prompt of 3 x 777 tokens
+              // through one 13B layer 1507 -> 1481 us, two additions of 14 each
+              if (residual != nullptr && m0 + epi_tid < M) {      // N % 8 == 0: a group of eight columns is inside or outside
+                const __nv_bfloat16* rp = residual + static_cast<int64_t>(m0 + epi_tid) * ldr + col0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  if (col0 + 8 * q < N) {
+                    const uint4 r4 = __ldg(reinterpret_cast<const uint4*>(rp) + q);
+                    const uint32_t w[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                      r[8 * q + 2 * e] = __float_as_uint(__uint_as_float(r[8 * q + 2 * e]) + __uint_as_float(w[e] << 16));
+                      r[8 * q + 2 * e + 1] = __float_as_uint(__uint_as_float(r[8 * q + 2 * e + 1]) + __uint_as_float(w[e] & 0xffff0000u));
+                    }
+                  }
+                }
+              }
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -418,7 +435,8 @@ static int max_clusters(int max_ctas) {
 
 template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G = 1>
 static int launch_variant(const Operands<G>& op, int groups, int M, int N, int mn3d, int* status, cudaStream_t stream, int max_ctas,
-                          int splits, const __nv_bfloat16* bias = nullptr, int act = 0) {
+                          int splits, const __nv_bfloat16* bias = nullptr, int act = 0, const __nv_bfloat16* residual = nullptr,
+                          int ldr = 0) {
   auto kfn = gemm2_bf16_kernel<A_MN, B_MN, EPI, TILE_N, G>;
   static bool configured = false;
   if (!configured) {
@@ -428,7 +446,7 @@ static int launch_variant(const Operands<G>& op, int groups, int M, int N, int m
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N) * splits * groups;
   int clusters = max_clusters(max_ctas);
   if (clusters > tiles) clusters = tiles;
-  kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(op, groups, M, N, mn3d, splits, status, bias, act);
+  kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(op, groups, M, N, mn3d, splits, status, bias, act, residual, ldr);
   return cudaGetLastError() == cudaSuccess ? kLaunchOk : kErrCuda;
 }
 
@@ -485,17 +503,18 @@ PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, in
   return kErrBadShape;
 }
 
-// C = act(A B + bias) (swiglu = 0; C bf16 [M, N]) or C = silu(gate) * up over interleaved (gate, up) column pairs
-// (swiglu = 1; C bf16 [M, N / 2], N a multiple of 16, bias must be null).  Operand layouts as pd_gemm_bf16_2cta.
+// C = act(A B + bias) + residual (swiglu = 0; C bf16 [M, N]; bias and residual may be null; with a residual N and ldr are multiples of
+// 8) or C = silu(gate) * up over interleaved (gate, up) column pairs (swiglu = 1; C bf16 [M, N / 2], N a multiple of 16, bias and
+// residual must be null).  Operand layouts as pd_gemm_bf16_2cta.
 PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                                    int a_mn_major, int b_mn_major, const void* bias, int act, int swiglu, int* status,
-                                    cudaStream_t stream) {
+                                    int a_mn_major, int b_mn_major, const void* bias, int act, int swiglu, const void* residual, int ldr,
+                                    int* status, cudaStream_t stream) {
   using namespace pd;
   using namespace pd::gemm2;
   if (M <= 0 || N <= 0 || K <= 0 || act < 0 || act > 4) return kErrBadShape;
-  if (swiglu && (bias != nullptr || (N % 16))) return kErrBadShape;
-  if (!aligned16(A) || !aligned16(B) || !aligned16(C)) return kErrAlignment;
-  if ((lda % 8) || (ldb % 8) || (ldc % 8)) return kErrAlignment;
+  if (swiglu && (bias != nullptr || residual != nullptr || (N % 16))) return kErrBadShape;
+  if (!aligned16(A) || !aligned16(B) || !aligned16(C) || !aligned16(residual)) return kErrAlignment;
+  if ((lda % 8) || (ldb % 8) || (ldc % 8) || (residual != nullptr && ((ldr % 8) || (N % 8)))) return kErrAlignment;
   const int TN = swiglu ? 256 : tile_n(M, N, 1, 0), BN_HALF = TN / 2;
   Operands<1> op;
   op.k[0] = K;
@@ -507,12 +526,12 @@ PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M
   else ok &= encode_tmap_mn(&op.b[0], B, N, K, uint64_t(ldb) * 2, BN_HALF / 64, BK, &b3d);
   ok &= encode_tmap_2d(&op.c[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, C, swiglu ? N / 2 : N, M, uint64_t(ldc) * 2, 64, BM);
   if (!ok) return kErrTensorMap;
-  const __nv_bfloat16* bp = static_cast<const __nv_bfloat16*>(bias);
+  const __nv_bfloat16 *bp = static_cast<const __nv_bfloat16*>(bias), *rp = static_cast<const __nv_bfloat16*>(residual);
 #define PD_GEMM2_EPI_CASE(AM, BM_)                                                                              \
   if (a_mn_major == AM && b_mn_major == BM_) {                                                                  \
     if (swiglu) return launch_variant<AM, BM_, kSwiglu, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1); \
-    return TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act) \
-                     : launch_variant<AM, BM_, kBiasAct, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act); \
+    return TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr) \
+                     : launch_variant<AM, BM_, kBiasAct, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr); \
   }
   PD_GEMM2_EPI_CASE(0, 0) PD_GEMM2_EPI_CASE(0, 1) PD_GEMM2_EPI_CASE(1, 0) PD_GEMM2_EPI_CASE(1, 1)
 #undef PD_GEMM2_EPI_CASE

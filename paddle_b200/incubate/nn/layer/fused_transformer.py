@@ -280,10 +280,12 @@ class FusedMultiTransformer(Layer):
             acc = ws[:M]
             native.gemm_splitk(x, w, acc, s)
             return native.splitk_finalize(acc, residual=residual)
+        if residual is None:
+            return native.gemm(x, w)
+        if native.GEMM_IMPL == "2cta" and w.shape[1] % 8 == 0 and native.rows16(residual):
+            return native.gemm_epilogue(x, w, residual=residual)
         y = native.gemm(x, w)
-        if residual is not None:
-            y = native.add_bf16(y, residual, out=y)
-        return y
+        return native.add_bf16(y, residual, out=y)
 
     def _all_reduce(self, t):
         if self._tp_group is not None:

@@ -293,3 +293,19 @@ def test_shape_keeping_operators_keep_the_distribution():
     sum(o.sum() for o in outs).backward()
     assert x.grad is not None and torch.isfinite(x.grad.float()).all()
     assert not K.rms_norm(paddle.to_tensor(torch.randn(4, 256, device="cuda").bfloat16()), w).is_dist()
+
+
+@pytest.mark.parametrize("M,N,K,act", [(100, 256, 128, None), (129, 264, 200, None), (300, 520, 256, "silu"), (2331, 640, 512, None)])
+def test_gemm_residual_epilogue(M, N, K, act):
+    """act(x W + b) + residual from the GEMM epilogue, edges of rows and columns, a residual with its own row stride."""
+    from paddle_b200.ops import _lib, native
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w, b, wide = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((M, K), (K, N), (N,), (M, N + 16)))
+    res = wide[:, 8:N + 8]
+    for bias in (None, b):
+        y = native.gemm_epilogue(x, w, bias, act, residual=res)
+        _lib.check_status()
+        h = x.float() @ w.float() + (0 if bias is None else bias.float())
+        ref = (torch.nn.functional.silu(h) if act else h) + res.float()
+        # one rounding to bf16; sums of K products in fp32 (both sides), 2^-6 for the fast exponential of the activation
+        assert ((y.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-3 + (2 ** -6 if act else 0)).all()
