@@ -119,7 +119,10 @@ __device__ __forceinline__ void tma2_load_3d(void* smem_dst, const CUtensorMap* 
 }
 
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
-  constexpr int G = 8;  // 256-row tiles per raster group: keeps a wave's A/B working set inside L2
+  // 256-row tiles per raster group: their rows of A stay in the L2 while the columns of B pass once.  Under sustained load (the power
+  // cap), us with 4 / 8 / 16 / 32: 4096 x 12288 x 4096 335 / 316 / 305 / -, its weight gradient 362 / 343 / 331 / -, 2331 x 27648 x
+  // 5120 - / 571 / 540 / 544, 8192 x 4096 x 4096 - / 214 / 210 / 224 (there the group's own rows no longer stay).
+  constexpr int G = 16;
   const int per_group = G * tiles_n;
   const int g = t / per_group;
   const int first_m = g * G;
