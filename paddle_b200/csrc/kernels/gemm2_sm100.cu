@@ -1,7 +1,7 @@
 // Two-SM (cta_group::2) variant of the persistent bf16 GEMM for sm_100a:  C[M,N] (=|+=) op(A)[M,K] * op(B)[K,N]
 //
-// A cluster of two CTAs (one SM pair) owns a 256 x TN output tile, TN = 256 or, for products whose tiles all run at once, 128
-// (tile_n below).  CTA r of the pair loads rows [128 r, 128 r + 128) of the A tile and columns [TN / 2 r, TN / 2 (r + 1)) of the
+// A cluster of two CTAs (one SM pair) owns a 256 x TN output tile, TN = 256, for products whose tiles all run at once 128, for deep
+// ones 512 in two accumulators of 256 columns (tile_n below).  CTA r of the pair loads rows [128 r, 128 r + 128) of the A tile and columns [TN / 2 r, TN / 2 (r + 1)) of the
 // B tile into ITS OWN shared memory (plain per-CTA TMA loads, no cluster multicast), so with TN = 256 every k-block costs each SM
 // 32 KB of shared-memory fill (six stages; 24 KB and eight stages with TN = 128) instead of the 48 KB of the 128 x 256
 // single-CTA tile, and the tensor core reads half of B from the partner SM.  One thread of the leader CTA (cluster rank 0; its MMA
@@ -15,6 +15,7 @@
 //   empty[s]  in both CTAs, released by tcgen05.commit.cta_group::2 with a CTA mask of both
 //   tfull[a]  in both CTAs, same commit form: accumulator a is complete
 //   tempty[a] leader only, 2 arrivals: each CTA's epilogue has drained its half of accumulator a
+// Accumulators alternate between tiles; those of a 512-column tile both belong to it.
 // Same operand-layout support, epilogues (bf16 store / fp32 store / fp32 reduce-add) and split-K slicing as
 // gemm_sm100.cu; replaces the cuBLAS call behind matmul / linear
 // (reference: paddle/phi/kernels/funcs/blas/blas_impl.cu.h:426).
@@ -29,8 +30,8 @@ constexpr int TILE_M = 256;
 constexpr int A_STAGE_BYTES = BM * BK * 2;        // 16 KB
 constexpr int C_CHUNK_BYTES = BM * 128;
 constexpr int NUM_THREADS = 192;
-// TN: columns of the pair's tile, 256 or 128; each CTA holds half of the B tile
-constexpr int stages(int tn) { return tn == 256 ? 6 : 8; }
+// TN: columns of the pair's tile, 512, 256 or 128; each CTA holds half of the B tile
+constexpr int stages(int tn) { return tn == 512 ? 4 : (tn == 256 ? 6 : 8); }
 constexpr int b_stage_bytes(int tn) { return tn / 2 * BK * 2; }
 constexpr int smem_bytes(int tn) { return stages(tn) * (A_STAGE_BYTES + b_stage_bytes(tn)) + 2 * C_CHUNK_BYTES + 1024 + 256; }
 constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;   // clears the CTA-pair bit of a shared::cluster address -> leader CTA
@@ -158,8 +159,10 @@ template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int N, int mn3d, int splits, int* status,
                   const __nv_bfloat16* bias, int act, const __nv_bfloat16* residual, int ldr) {
-  constexpr int STAGES = stages(TILE_N), BN_HALF = TILE_N / 2, B_STAGE_BYTES = b_stage_bytes(TILE_N);
-  constexpr uint32_t TM_COLS = 2 * TILE_N;
+  // accumulators hold ACC_N columns; a 512-column tile takes both of one tile, narrower ones alternate between tiles
+  constexpr int ACC_N = TILE_N == 512 ? 256 : TILE_N, HALVES = TILE_N / ACC_N;
+  constexpr int STAGES = stages(TILE_N), BN_HALF = ACC_N / 2, B_STAGE_BYTES = b_stage_bytes(TILE_N), B_HALF_BYTES = B_STAGE_BYTES / HALVES;
+  constexpr uint32_t TM_COLS = 2 * ACC_N;
   extern __shared__ uint8_t smem_raw[];
   // the dynamic shared memory starts at the same offset in both CTAs, so the aligned carve-up is identical in both
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -179,6 +182,8 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
   const int num_tiles = group_tiles * (G == 1 ? 1 : groups);
   // tile t: which product it belongs to, its number in that one, its blocks of K
   auto group_of = [&](int t) { return G == 1 ? 0 : t / group_tiles; };
+  // accumulators of a tile that starts at column n0: the second half of a wide one may lie outside the matrix
+  auto halves_at = [&](int n0) { return HALVES == 2 && n0 + ACC_N < N ? 2 : 1; };
   auto k_range = [&](int g, int t, int& kb0, int& kb1) {
     const int kb_total = (op.k[g] + BK - 1) / BK, kbs = (kb_total + splits - 1) / splits;
     kb0 = (t % splits) * kbs;
@@ -220,14 +225,16 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
         const int g = group_of(t), tg = t - g * group_tiles;
         tile_coords(tg / splits, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * TILE_M + static_cast<int>(cta_rank) * BM;
-        const int n0 = tn * TILE_N + static_cast<int>(cta_rank) * BN_HALF;
+        const int n0 = tn * TILE_N + static_cast<int>(cta_rank) * BN_HALF, halves = halves_at(tn * TILE_N);
         k_range(g, tg, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&bars->empty[s], ph ^ 1, abort_flag, status, 100 + s)) { ok = false; break; }
-          if (leader) mbar_expect_tx(&bars->full[s], 2 * (A_STAGE_BYTES + B_STAGE_BYTES));
+          if (leader) mbar_expect_tx(&bars->full[s], 2 * (A_STAGE_BYTES + halves * B_HALF_BYTES));
           const int k0 = kb * BK;
           load_half<A_MN, BM>(sA + s * A_STAGE_BYTES, &op.a[g], &bars->full[s], m0, k0, (mn3d & 1) != 0);
           load_half<B_MN, BN_HALF>(sB + s * B_STAGE_BYTES, &op.b[g], &bars->full[s], n0, k0, (mn3d & 2) != 0);
+          if (HALVES == 2 && halves == 2)
+            load_half<B_MN, BN_HALF>(sB + s * B_STAGE_BYTES + B_HALF_BYTES, &op.b[g], &bars->full[s], n0 + ACC_N, k0, (mn3d & 2) != 0);
           ++issued;
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
@@ -242,7 +249,7 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
     if (leader) {
       const uint32_t lead = elect_one() ? 1u : 0u;
       const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
-      constexpr uint32_t idesc = make_idesc(TILE_M, TILE_N, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc(TILE_M, ACC_N, A_MN, B_MN);
       constexpr uint32_t a_kstep = A_MN ? 2048u : 32u;
       constexpr uint32_t b_kstep = B_MN ? 2048u : 32u;
       constexpr uint32_t a_lbo = A_MN ? 8192u : 16u;
@@ -252,12 +259,63 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
+      if (HALVES == 2) {
+        // A batch of K blocks goes into the first accumulator, then into the second.  The first and last batch of a tile are all
+        // stages long: the first accumulator is drained under the end of its tile, the second under the beginning of the next.
+        int it1 = 0;                                                             // tiles with two halves so far
+        for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {
+          const int g = group_of(t), tg = t - g * group_tiles;
+          int tm_, tn, kb0, kb1;
+          tile_coords(tg / splits, tiles_m, tiles_n, tm_, tn);
+          k_range(g, tg, kb0, kb1);
+          const int halves = halves_at(tn * TILE_N);
+          if (!mbar_wait_warp(&bars->tempty[0], (it & 1) ^ 1, abort_flag, status, 200)) { ok = false; break; }
+          bool first = true;
+#pragma unroll 1
+          for (int left = kb1 - kb0; left > 0 && ok;) {
+            const int n = first || left <= STAGES ? min(STAGES, left) : 1;
+            int si = s;
+            uint32_t phi = ph;
+#pragma unroll 1
+            for (int i = 0; i < n; ++i) {
+              if (!mbar_wait_warp(&bars->full[si], phi, abort_flag, status, 300 + si)) { ok = false; break; }
+              tc_fence_after();
+              const uint64_t ad = a_desc0 + si * (A_STAGE_BYTES >> 4), bd = b_desc0 + si * (B_STAGE_BYTES >> 4);
+#pragma unroll
+              for (int k = 0; k < BK / 16; ++k)
+                umma2_bf16_ss_if(lead, tm, ad + k * (a_kstep >> 4), bd + k * (b_kstep >> 4), idesc, !first || (i | k) != 0 ? 1u : 0u);
+              if (++si == STAGES) si = 0, phi ^= 1;
+            }
+            if (!ok) break;
+            if (n == left) umma2_commit_both_if(lead, &bars->tfull[0]);
+            if (first && halves == 2) {
+              if (!mbar_wait_warp(&bars->tempty[1], (it1 & 1) ^ 1, abort_flag, status, 201)) { ok = false; break; }
+              tc_fence_after();
+            }
+#pragma unroll 1
+            for (int i = 0; i < n; ++i) {
+              const uint64_t ad = a_desc0 + s * (A_STAGE_BYTES >> 4), bd = b_desc0 + ((s * B_STAGE_BYTES + B_HALF_BYTES) >> 4);
+              if (halves == 2) {
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k)
+                  umma2_bf16_ss_if(lead, tm + ACC_N, ad + k * (a_kstep >> 4), bd + k * (b_kstep >> 4), idesc, !first || (i | k) != 0 ? 1u : 0u);
+              }
+              umma2_commit_both_if(lead, &bars->empty[s]);
+              if (++s == STAGES) s = 0, ph ^= 1;
+            }
+            if (n == left && halves == 2) umma2_commit_both_if(lead, &bars->tfull[1]);
+            left -= n;
+            first = false;
+          }
+          it1 += halves - 1;
+        }
+      } else
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {
         const int acc = it & 1;
         const uint32_t acc_ph = (it >> 1) & 1;
         if (!mbar_wait_warp(&bars->tempty[acc], acc_ph ^ 1, abort_flag, status, 200 + acc)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tm + acc * TILE_N;
+        const uint32_t d_tmem = tm + acc * ACC_N;
         const int g = group_of(t);
         int kb0, kb1;
         k_range(g, t - g * group_tiles, kb0, kb1);
@@ -285,26 +343,32 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
     // ------------------------------------------------------------ epilogue (warps 0..3 of each CTA: its 128 rows)
     const int epi_tid = threadIdx.x;
     constexpr int CW = (EPI == kStoreBf16 || EPI == kBiasAct) ? 64 : (EPI == kSwiglu ? 128 : 32);
-    constexpr int NCHUNK = TILE_N / CW;
+    constexpr int NCHUNK = ACC_N / CW;
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const bool bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
     int it = 0;
     int chunk_counter = 0;
-    for (int t = cluster_id; t < num_tiles; t += n_clusters, ++it) {
+    int it1 = 0;                              // wide tiles with two halves so far
+    bool live = true;
+    for (int t = cluster_id; t < num_tiles && live; t += n_clusters, ++it) {
       int tm, tn;
       const int g = group_of(t);
       tile_coords((t - g * group_tiles) / splits, tiles_m, tiles_n, tm, tn);
-      const int m0 = tm * TILE_M + static_cast<int>(cta_rank) * BM, n0 = tn * TILE_N;
-      const int acc = it & 1;
-      const uint32_t acc_ph = (it >> 1) & 1;
+      const int m0 = tm * TILE_M + static_cast<int>(cta_rank) * BM;
+      const int halves = halves_at(tn * TILE_N);
+#pragma unroll 1
+      for (int half = 0; half < halves; ++half) {
+      const int n0 = tn * TILE_N + half * ACC_N;
+      const int acc = HALVES == 2 ? half : it & 1;
+      const uint32_t acc_ph = HALVES == 2 ? (half == 0 ? it : it1) & 1 : (it >> 1) & 1;
       if (epi_tid == 0) {
         const bool ok = mbar_wait(&bars->tfull[acc], acc_ph, abort_flag, status, 400 + acc);
         bars->epi_decision = ok ? 1 : 0;
       }
       named_bar_sync(1, 128);
-      if (bars->epi_decision == 0) break;
+      if (bars->epi_decision == 0) { live = false; break; }
       tc_fence_after();
-      const uint32_t t_acc = tmem_base + lane_base + acc * TILE_N;
+      const uint32_t t_acc = tmem_base + lane_base + acc * ACC_N;
       const bool rows_live = m0 < M;          // a partner half entirely below the matrix stores nothing
 #pragma unroll 1
       for (int c = 0; c < NCHUNK; ++c, ++chunk_counter) {
@@ -419,6 +483,8 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
           tma_commit_group();
         }
       }
+      }
+      it1 += halves - 1;
     }
     if (epi_tid == 0) tma_wait_group<0>();
   }
@@ -453,11 +519,19 @@ static int launch_variant(const Operands<G>& op, int groups, int M, int N, int m
   return cudaGetLastError() == cudaSuccess ? kLaunchOk : kErrCuda;
 }
 
-// 256 x 128 tiles when even those all run at once on the pairs that the call may use: every pair then does half the work of a 256 x 256 tile (us, wide / narrow:
-// 512 x 1024 x 512 15.3 / 13.3, 818 x 616 x 3064 35.8 / 31.7, 200 x 4096 x 4096 34.8 / 29.7).  With more tiles the wide form wins
+// 256 x 128 tiles when even those all run at once on the pairs that the call may use: every pair then does half the work of a 256 x 256 tile (us, 256 / 128:
+// 512 x 1024 x 512 15.3 / 13.3, 818 x 616 x 3064 35.8 / 31.7, 200 x 4096 x 4096 34.8 / 29.7).  With more tiles the other form wins
 // although its last wave is emptier: a 64-deep block of a narrow tile is 256 tensor cycles and costs some 350 (4096^3: 96 / 124;
 // 1000 x 11008 x 4096, 3 waves against 2.5: 84 / 109).
-static int tile_n(int M, int N, int splits, int max_ctas) {
+//
+// 256 x 512 tiles for deep products (K >= 8192) where they take no more rounds: a K block then brings 48 KB to an SM for the MMAs that
+// two 256 x 256 tiles bring 64 KB for, and at the power cap that is time (without any loads of B the same products ran 10 to 12 %
+// faster).  us under sustained load, 256 / 512 columns, groups of 16 row tiles: 4096 x 4096 x 12288 345 / 322, x 22016 610 / 571,
+// x 32000 892 / 855, x 11008 311 / 290, x 8192 (into fp32) 238 / 228; but x 4096 111 / 112, and where the rounds come out longer 2331 x
+// 5120 x 13824 290 / 321, 8192 x 4096 x 4096 210 / 224.
+static int tile_n(int M, int N, int K, int splits, int max_ctas) {
+  const int64_t rows = (M + TILE_M - 1) / TILE_M, pairs = max_clusters(max_ctas);
+  if (K >= 8192 && splits == 1 && 2 * ((rows * ((N + 511) / 512) + pairs - 1) / pairs) <= (rows * ((N + 255) / 256) + pairs - 1) / pairs) return 512;
   return static_cast<int64_t>((M + TILE_M - 1) / TILE_M) * ((N + 127) / 128) * splits <= max_clusters(max_ctas) ? 128 : 256;
 }
 
@@ -465,7 +539,8 @@ static int tile_n(int M, int N, int splits, int max_ctas) {
 }  // namespace pd
 
 // Columns of the tiles that pd_gemm_bf16_2cta works in.
-PD_EXPORT int pd_gemm_2cta_tile_n(int M, int N, int splits, int max_ctas) { return pd::gemm2::tile_n(M, N, splits, max_ctas); }
+PD_EXPORT int pd_gemm_2cta_tile_n(int M, int N, int splits, int max_ctas) { return pd::gemm2::tile_n(M, N, 0, splits, max_ctas); }   // shallow ones
+PD_EXPORT int pd_gemm_2cta_tile_n_at(int M, int N, int K, int splits, int max_ctas) { return pd::gemm2::tile_n(M, N, K, splits, max_ctas); }
 
 // Same contract as pd_gemm_bf16 / pd_gemm_bf16_splitk (gemm_sm100.cu); splits = 1 for the plain form.
 PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
@@ -483,7 +558,7 @@ PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, in
   }
   if (!aligned16(A) || !aligned16(B) || !aligned16(C)) return kErrAlignment;
   if ((lda % 8) || (ldb % 8) || (epi == kStoreBf16 ? (ldc % 8) : (ldc % 4))) return kErrAlignment;
-  const int TN = tile_n(M, N, splits, max_ctas), BN_HALF = TN / 2;
+  const int TN = tile_n(M, N, K, splits, max_ctas), BN_HALF = TN == 512 ? 128 : TN / 2;
   Operands<1> op;
   op.k[0] = K;
   bool ok = true;
@@ -497,7 +572,8 @@ PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, in
   if (!ok) return kErrTensorMap;
 #define PD_GEMM2_CASE(AM, BM_, E)                                                                  \
   if (a_mn_major == AM && b_mn_major == BM_ && epi == E)                                           \
-    return TN == 128 ? launch_variant<AM, BM_, E, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, max_ctas, splits) \
+    return TN == 512 ? launch_variant<AM, BM_, E, 512>(op, 1, M, N, a3d | (b3d << 1), status, stream, max_ctas, splits) \
+         : TN == 128 ? launch_variant<AM, BM_, E, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, max_ctas, splits) \
                      : launch_variant<AM, BM_, E, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, max_ctas, splits);
   PD_GEMM2_CASE(0, 0, 0) PD_GEMM2_CASE(0, 1, 0) PD_GEMM2_CASE(1, 0, 0) PD_GEMM2_CASE(1, 1, 0)
   PD_GEMM2_CASE(0, 0, 1) PD_GEMM2_CASE(0, 1, 1) PD_GEMM2_CASE(1, 0, 1) PD_GEMM2_CASE(1, 1, 1)
@@ -518,7 +594,7 @@ PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M
   if (swiglu && (bias != nullptr || residual != nullptr || (N % 16))) return kErrBadShape;
   if (!aligned16(A) || !aligned16(B) || !aligned16(C) || !aligned16(residual)) return kErrAlignment;
   if ((lda % 8) || (ldb % 8) || (ldc % 8) || (residual != nullptr && ((ldr % 8) || (N % 8)))) return kErrAlignment;
-  const int TN = swiglu ? 256 : tile_n(M, N, 1, 0), BN_HALF = TN / 2;
+  const int TN = swiglu ? 256 : tile_n(M, N, K, 1, 0), BN_HALF = TN == 512 ? 128 : TN / 2;
   Operands<1> op;
   op.k[0] = K;
   bool ok = true;
@@ -533,7 +609,8 @@ PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M
 #define PD_GEMM2_EPI_CASE(AM, BM_)                                                                              \
   if (a_mn_major == AM && b_mn_major == BM_) {                                                                  \
     if (swiglu) return launch_variant<AM, BM_, kSwiglu, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1); \
-    return TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr) \
+    return TN == 512 ? launch_variant<AM, BM_, kBiasAct, 512>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr) \
+         : TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr) \
                      : launch_variant<AM, BM_, kBiasAct, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr); \
   }
   PD_GEMM2_EPI_CASE(0, 0) PD_GEMM2_EPI_CASE(0, 1) PD_GEMM2_EPI_CASE(1, 0) PD_GEMM2_EPI_CASE(1, 1)
@@ -564,7 +641,7 @@ PD_EXPORT int pd_gemm_bf16_grouped_tn(const void* A, const void* B, void* C, con
   int64_t below_rows = INT64_MAX;      // of the product taken last; equal ones are taken in their order
   int below_g = -1;
   while (left > 0) {
-    const int n = left < MAX_GROUPS ? left : MAX_GROUPS, TN = tile_n(M, N, n, 0);
+    const int n = left < MAX_GROUPS ? left : MAX_GROUPS, TN = tile_n(M, N, 0, n, 0);
     int a3d = 0, b3d = 0;
     bool ok = true;
     for (int i = 0; i < n; ++i) {

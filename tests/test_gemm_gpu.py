@@ -175,3 +175,31 @@ def test_gemm_grouped_weight_gradients(M, N, counts):
             assert ((plain[g].float() - ref).abs() <= 2 ** -8 * ref.abs() + tol).all()
         else:
             assert torch.equal(plain[g], torch.full_like(plain[g], 7.0))
+
+
+@pytest.mark.parametrize("M,N,K_,max_ctas,width", [(304, 776, 8200, 2, 512), (200, 1112, 8256, 8, 512), (304, 776, 8136, 2, 256), (304, 520, 8200, 2, 256),
+                                                   (2048, 2600, 8200, 0, 512)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+def test_deep_products_take_wide_tiles(M, N, K_, max_ctas, width, ta, tb):
+    """256 x 512 tiles, the last one with its second half full, partly or wholly outside, all layouts and epilogues, and shapes just
+    outside the rule; the same sums in the same order as the other tiles."""
+    from paddle_b200.ops import _lib, native
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _lib.kernels().pd_gemm_2cta_tile_n_at(M, N, K_, 1, max_ctas) == width
+    g = torch.Generator(device="cuda").manual_seed(M + N + K_)
+    a = torch.randn((K_, M) if ta else (M, K_), device="cuda", generator=g).bfloat16()
+    b = torch.randn((N, K_) if tb else (K_, N), device="cuda", generator=g).bfloat16()
+    bias = torch.randn(N, device="cuda", generator=g).bfloat16()
+    ref = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    # The tensor cores cut off what does not fit when they add: each of K_ / 16 steps loses up to 2^-23 of a running sum, which for
+    # products of size 1 stays below 5 sqrt(K_).  Then one rounding to bf16.
+    sums = K_ / 16 * 5 * K_ ** 0.5 * 2 ** -23
+    tol = ref.abs() * 2 ** -8 + sums
+    assert (native.gemm(a, b, ta, tb, max_ctas=max_ctas).double() - ref).abs().le(tol).all()
+    assert (native.gemm(a, b, ta, tb, out_dtype=torch.float32, max_ctas=max_ctas).double() - ref).abs().max() <= sums
+    acc = torch.randn(M, N, device="cuda", generator=g)
+    got = native.gemm(a, b, ta, tb, out=acc.clone(), accumulate=True, max_ctas=max_ctas)
+    assert (got.double() - ref - acc.double()).abs().max() <= sums + 1e-4
+    assert (native.gemm_epilogue(a, b, bias, None, ta, tb).double() - ref - bias.double()).abs().le(tol + bias.double().abs() * 2 ** -8).all()
+    torch.cuda.synchronize()
+    _lib.check_status()
