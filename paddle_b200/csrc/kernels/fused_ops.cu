@@ -384,16 +384,19 @@ __global__ void __launch_bounds__(32 * CS_ROWS) column_sum_kernel(const float* _
 }
 
 // Sums over the rows of a bf16 matrix (bias gradients): a block takes 64 columns (8 lanes of 8) and every gridDim.y-th group of
-// 32 rows; with one block row the sums are the result, otherwise they go to partial[gridDim.y][N] for column_sum_kernel.
-__global__ void __launch_bounds__(256) bf16_row_sum_kernel(const bf16* __restrict__ x, int64_t ld, bf16* __restrict__ out,
+// 64 rows; with one block row the sums are the result, otherwise they go to partial[gridDim.y][N] for column_sum_kernel.
+// Latency: with 256 threads and four loads each in flight 1000 x 11008 took 14.7 us after a product and 8192 x 11008 88, 10.6 and 50 with twice
+// the threads and loads.
+constexpr int RS_ROWS = 64;
+__global__ void __launch_bounds__(8 * RS_ROWS) bf16_row_sum_kernel(const bf16* __restrict__ x, int64_t ld, bf16* __restrict__ out,
                                                            float* __restrict__ partial, int64_t rows, int N) {
-  __shared__ float red[32][65];
+  __shared__ float red[RS_ROWS][65];
   const int v = threadIdx.x & 7, g = threadIdx.x >> 3;
   const int c = blockIdx.x * 64 + v * 8;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (c < N) {
-#pragma unroll 4
-    for (int64_t r = static_cast<int64_t>(blockIdx.y) * 32 + g; r < rows; r += static_cast<int64_t>(gridDim.y) * 32) {
+#pragma unroll 8
+    for (int64_t r = static_cast<int64_t>(blockIdx.y) * RS_ROWS + g; r < rows; r += static_cast<int64_t>(gridDim.y) * RS_ROWS) {
       float f[8];
       load8(x + r * ld + c, f);
 #pragma unroll
@@ -407,7 +410,7 @@ __global__ void __launch_bounds__(256) bf16_row_sum_kernel(const bf16* __restric
   if (threadIdx.x < 64 && col < N) {
     float s = 0.f;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) s += red[k][threadIdx.x];
+    for (int k = 0; k < RS_ROWS; ++k) s += red[k][threadIdx.x];
     if (partial != nullptr) partial[static_cast<size_t>(blockIdx.y) * N + col] = s;
     else out[col] = __float2bfloat16(s);
   }
@@ -1035,7 +1038,7 @@ PD_EXPORT int pd_bf16_row_sum(const void* x, int64_t ld, void* out, float* parti
   if (!aligned16(x)) return kErrAlignment;
   const int parts = pd_bf16_row_sum_parts(rows, N);
   if (parts > 1 && partial == nullptr) return kErrBadShape;
-  bf16_row_sum_kernel<<<dim3((N + 63) / 64, parts), 256, 0, stream>>>((const bf16*)x, ld, (bf16*)out, parts > 1 ? partial : nullptr, rows, N);
+  bf16_row_sum_kernel<<<dim3((N + 63) / 64, parts), 8 * RS_ROWS, 0, stream>>>((const bf16*)x, ld, (bf16*)out, parts > 1 ? partial : nullptr, rows, N);
   if (parts > 1) column_sum_kernel<bf16><<<(N + 31) / 32, 32 * CS_ROWS, 0, stream>>>(partial, (bf16*)out, parts, N, 0);
   return PD_CHECK_LAUNCH();
 }
