@@ -20,6 +20,7 @@
 // with split-K atomics and a finalising kernel each: 123 us).  Two 7B layers and the head for one sequence, 1.07 GB of weights
 // (161 us at the copy rate): 382 -> 262 us, with the qkv epilogue, dependent launches and a CTA per row in the norms 216 us;
 // two 13B layers and the head, batch 64, 842 -> 760 -> 717 us (attention 387 of it, at the copy rate).
+// Weights that leave the L2 first and cuts of K into eight for few rows: 215 -> 212 and 712 -> 707 us.
 #include "host_utils.h"
 #include "sm100_prims.cuh"
 
@@ -140,6 +141,10 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 4) {
     if (lane == 0) {
+      // Large weights pass through the L2 without pushing out x and the cached keys (us, normal / first to leave: 64 rows 5120 x 15360
+      // 28.8 / 27.3, 5120 x 32000 52.1 / 49.9, 13824 x 5120 29.7 / 28.9, 128 rows 4096 x 22016 38.8 / 37.0, one row 28.8 / 28.6).  The
+      // layers of a model with small ones may fit the L2 from token to token, so those stay.
+      const uint64_t policy = l2_policy(static_cast<int64_t>(p.K) * p.N * 2 >= (int64_t(40) << 20));
       prefetch_tmap(&tmW);
       prefetch_tmap(&tmX);
       bool ok = true;
@@ -147,8 +152,8 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       auto arm_and_load_w = [&](int i) {
         const int s = i % ST, k0 = (kb0 + i) * BK;
         mbar_expect_tx(&bars->full[s], W_STAGE_BYTES + XB);
-        tma_load_2d(sW + s * W_STAGE_BYTES, &tmW, &bars->full[s], n0, k0);
-        tma_load_2d(sW + s * W_STAGE_BYTES + W_STAGE_BYTES / 2, &tmW, &bars->full[s], n1, k0);
+        tma_load_2d(sW + s * W_STAGE_BYTES, &tmW, &bars->full[s], n0, k0, policy);
+        tma_load_2d(sW + s * W_STAGE_BYTES + W_STAGE_BYTES / 2, &tmW, &bars->full[s], n1, k0, policy);
       };
       const int ahead = p.weights_ready ? min(nk, ST) : 0;
       for (int i = 0; i < ahead; ++i) arm_and_load_w(i);
@@ -298,10 +303,11 @@ static int setup(const void* x, const void* w, int M, int N, int K, int ldx, int
     return kErrTensorMap;
   const int kb = (K + BK - 1) / BK;
   if (splits == 0) {
-    // two CTAs per SM in one wave, no CTA with fewer than four blocks of K; at most 4: with 8 the partial tiles cost more
-    // than the further loads in flight bring (K = N = 4096, M = 1 / 64 / 128: 16.3 / 18.6 / 22.5 us with 4, 16.4 / 22.5 / 29 with 8)
+    // two CTAs per SM in one wave, no CTA with fewer than four blocks of K; from nine rows on at most 4: with 8 the partial tiles
+    // cost more than the further loads in flight bring (us with 4 / 8: K = N = 4096, M = 1 8.7 / 7.7, 128 14.0 / 20.7; K = 11008,
+    // N = 4096, M = 1 16.9 / 15.8, 32 18.9 / 19.5)
     splits = 1;
-    while (splits < 4 && tiles * splits * 2 <= 2 * sm_count() && kb >= 8 * splits) splits *= 2;
+    while (splits < (M <= 8 ? MAX_SPLIT : 4) && tiles * splits * 2 <= 2 * sm_count() && kb >= 8 * splits) splits *= 2;
   }
   p->M = M;
   p->N = N;
