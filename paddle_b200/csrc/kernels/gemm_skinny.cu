@@ -142,9 +142,11 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (warp == 4) {
     if (lane == 0) {
       // Large weights pass through the L2 without pushing out x and the cached keys (us, normal / first to leave: 64 rows 5120 x 15360
-      // 28.8 / 27.3, 5120 x 32000 52.1 / 49.9, 13824 x 5120 29.7 / 28.9, 128 rows 4096 x 22016 38.8 / 37.0, one row 28.8 / 28.6).  The
-      // layers of a model with small ones may fit the L2 from token to token, so those stay.
-      const uint64_t policy = l2_policy(static_cast<int64_t>(p.K) * p.N * 2 >= (int64_t(40) << 20));
+      // 28.8 / 27.3, 5120 x 32000 52.1 / 49.9, 13824 x 5120 29.7 / 28.9, 128 rows 4096 x 22016 38.8 / 37.0, one row 28.8 / 28.6).  A model
+      // whose weights are all smaller than this may fit the L2 (126 MB) from token to token, so those stay: with 40 MB as the line one
+      // layer of 1024 and its 65 MB head took 49.1 instead of 47.2.
+      const bool pass_through = static_cast<int64_t>(p.K) * p.N * 2 >= (int64_t(72) << 20);
+      const uint64_t policy = l2_evict_first();
       prefetch_tmap(&tmW);
       prefetch_tmap(&tmX);
       bool ok = true;
@@ -152,8 +154,14 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       auto arm_and_load_w = [&](int i) {
         const int s = i % ST, k0 = (kb0 + i) * BK;
         mbar_expect_tx(&bars->full[s], W_STAGE_BYTES + XB);
-        tma_load_2d(sW + s * W_STAGE_BYTES, &tmW, &bars->full[s], n0, k0, policy);
-        tma_load_2d(sW + s * W_STAGE_BYTES + W_STAGE_BYTES / 2, &tmW, &bars->full[s], n1, k0, policy);
+        uint8_t* dst = sW + s * W_STAGE_BYTES;
+        if (pass_through) {
+          tma_load_2d(dst, &tmW, &bars->full[s], n0, k0, policy);
+          tma_load_2d(dst + W_STAGE_BYTES / 2, &tmW, &bars->full[s], n1, k0, policy);
+        } else {
+          tma_load_2d(dst, &tmW, &bars->full[s], n0, k0);
+          tma_load_2d(dst + W_STAGE_BYTES / 2, &tmW, &bars->full[s], n1, k0);
+        }
       };
       const int ahead = p.weights_ready ? min(nk, ST) : 0;
       for (int i = 0; i < ahead; ++i) arm_and_load_w(i);

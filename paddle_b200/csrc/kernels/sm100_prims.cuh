@@ -277,11 +277,11 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// The same with an L2 policy: how soon the lines may leave again.
-__device__ __forceinline__ uint64_t l2_policy(bool leaves_first) {
+// The same with an L2 policy: lines that leave again first.  (A load that names the normal policy is not one without: the products of
+// gemm2_sm100.cu took 2 % longer with it.)
+__device__ __forceinline__ uint64_t l2_evict_first() {
   uint64_t p;
-  if (leaves_first) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* tmap, uint64_t* bar, int x, int y, uint64_t policy) {
