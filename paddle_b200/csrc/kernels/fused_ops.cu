@@ -583,15 +583,20 @@ __global__ void rope_kernel(const bf16* __restrict__ x, bf16* __restrict__ out,
   }
 }
 
-// half_style for head dims whose 8-pair vectors divide a block: a block takes one token after the other, a thread keeps its
-// cos / sin values for all heads, and no index is divided.  (4096 tokens x 64 heads x 128: 47 us with the general kernel.)
+// half_style for head dims whose 8-pair vectors divide a block: `team` threads take one token after the other, a thread keeps its
+// vector of the tables for all heads that it rotates, has four heads in flight and divides no index.  The tables are fp32 and read by
+// every group of heads of a token, so a whole block for each token read more of them than of x (us, 256 / 64 threads a token: 4096
+// tokens of 64 heads 35.0 / 28.8, 2331 of 80 24.8 / 17.2, 3000 of 40 20.4 / 14.5, 16384 of 64 118 / 92; but 64 of 64 4.5 / 6.4, see
+// pd_rope).
 __global__ void __launch_bounds__(256) rope_half_kernel(const bf16* __restrict__ x, bf16* __restrict__ out, const float* __restrict__ cos_t,
                                                         const float* __restrict__ sin_t, const int64_t* __restrict__ position_ids,
                                                         int tokens, int heads, int D, int64_t token_stride, int64_t out_token_stride,
-                                                        int seq_len, float sin_sign) {
-  const int vph = D >> 4, v = threadIdx.x % vph, h0 = threadIdx.x / vph, hstep = 256 / vph;
+                                                        int seq_len, float sin_sign, int team) {
+  constexpr int U = 4;
+  const int vph = D >> 4, l = threadIdx.x % team, per_cta = 256 / team;
+  const int v = l % vph, h0 = l / vph, hstep = team / vph;
   const int i0 = v * 8, i1 = i0 + (D >> 1);
-  for (int tok = blockIdx.x; tok < tokens; tok += gridDim.x) {
+  for (int64_t tok = static_cast<int64_t>(blockIdx.x) * per_cta + threadIdx.x / team; tok < tokens; tok += static_cast<int64_t>(gridDim.x) * per_cta) {
     const int64_t pos = position_ids ? position_ids[tok] : tok % seq_len;
     float ca[8], sa[8], cb[8], sb[8];
     load8(cos_t + pos * D + i0, ca);
@@ -605,18 +610,31 @@ __global__ void __launch_bounds__(256) rope_half_kernel(const bf16* __restrict__
     }
     const bf16* src = x + tok * token_stride;
     bf16* dst = out + tok * out_token_stride;
-#pragma unroll 2
-    for (int h = h0; h < heads; h += hstep) {
-      float a[8], b[8], oa[8], ob[8];
-      load8(src + h * D + i0, a);
-      load8(src + h * D + i1, b);
+    for (int h = h0; h < heads; h += U * hstep) {
+      uint4 ra[U], rb[U];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        oa[j] = a[j] * ca[j] - b[j] * sa[j];
-        ob[j] = b[j] * cb[j] + a[j] * sb[j];
+      for (int k = 0; k < U; ++k) {
+        if (h + k * hstep < heads) {
+          ra[k] = *reinterpret_cast<const uint4*>(src + (h + k * hstep) * D + i0);
+          rb[k] = *reinterpret_cast<const uint4*>(src + (h + k * hstep) * D + i1);
+        }
       }
-      store8(dst + h * D + i0, oa);
-      store8(dst + h * D + i1, ob);
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        if (h + k * hstep < heads) {
+          const uint32_t wa[4] = {ra[k].x, ra[k].y, ra[k].z, ra[k].w}, wb[4] = {rb[k].x, rb[k].y, rb[k].z, rb[k].w};
+          float oa[8], ob[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float a = __uint_as_float((j & 1) ? (wa[j >> 1] & 0xffff0000u) : (wa[j >> 1] << 16));
+            const float b = __uint_as_float((j & 1) ? (wb[j >> 1] & 0xffff0000u) : (wb[j >> 1] << 16));
+            oa[j] = a * ca[j] - b * sa[j];
+            ob[j] = b * cb[j] + a * sb[j];
+          }
+          store8(dst + (h + k * hstep) * D + i0, oa);
+          store8(dst + (h + k * hstep) * D + i1, ob);
+        }
+      }
     }
   }
 }
@@ -947,9 +965,12 @@ PD_EXPORT int pd_rope(const void* x, void* out, const float* cos_t, const float*
                       int backward, cudaStream_t stream) {
   if (D % 16 != 0 || tokens <= 0 || (token_stride % 8) || (out_token_stride % 8)) return kErrBadShape;
   if (half_style && 256 % (D >> 4) == 0 && tokens <= INT32_MAX) {
-    const int blocks = tokens < 16 * sm_count() ? static_cast<int>(tokens) : 16 * sm_count();
+    // fewer tokens than two an SM: a whole block each
+    const int vph = D >> 4, team = tokens < 2 * sm_count() ? 256 : (vph > 64 ? vph : 64), per_cta = 256 / team;
+    const int64_t need = (tokens + per_cta - 1) / per_cta;
+    const int blocks = need < 16 * sm_count() ? static_cast<int>(need) : 16 * sm_count();
     rope_half_kernel<<<blocks, 256, 0, stream>>>((const bf16*)x, (bf16*)out, cos_t, sin_t, position_ids, static_cast<int>(tokens),
-                                                 heads, D, token_stride, out_token_stride, seq_len, backward ? -1.f : 1.f);
+                                                 heads, D, token_stride, out_token_stride, seq_len, backward ? -1.f : 1.f, team);
     return PD_CHECK_LAUNCH();
   }
   const int64_t work = tokens * heads * (D >> 4);

@@ -309,3 +309,25 @@ def test_gemm_residual_epilogue(M, N, K, act):
         ref = (torch.nn.functional.silu(h) if act else h) + res.float()
         # one rounding to bf16; sums of K products in fp32 (both sides), 2^-6 for the fast exponential of the activation
         assert ((y.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-3 + (2 ** -6 if act else 0)).all()
+
+
+@pytest.mark.parametrize("tokens", [1, 295, 296, 1203])
+@pytest.mark.parametrize("heads,D", [(1, 128), (5, 128), (33, 128), (9, 64), (3, 2048)])
+def test_rope_whole_blocks_and_teams(tokens, heads, D):
+    """Few tokens (a block each) and many (teams of threads), heads that do not divide among them, in place on a strided view, both
+    directions."""
+    from paddle_b200.ops import _lib, native
+    g = torch.Generator(device="cuda").manual_seed(tokens + heads)
+    buf = torch.randn(tokens, heads + 2, D, device="cuda", generator=g).bfloat16()
+    x = buf[:, :heads]
+    cos, sin = (torch.randn(tokens, D, device="cuda", generator=g) for _ in range(2))
+    xf, h, kept = x.float().clone(), D // 2, buf[:, heads:].clone()
+    for backward in (False, True):
+        sg = -sin if backward else sin
+        ref = torch.cat([xf[..., :h] * cos[:, None, :h] - xf[..., h:] * sg[:, None, :h],
+                         xf[..., h:] * cos[:, None, h:] + xf[..., :h] * sg[:, None, h:]], -1)
+        y = native.rope(x.unsqueeze(0), cos, sin, backward=backward)[0]
+        assert ((y.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-5).all()       # fp32 products, one rounding to bf16
+    native.rope(x.unsqueeze(0), cos, sin, out=x.unsqueeze(0), backward=True)
+    _lib.check_status()
+    assert torch.equal(x, y) and torch.equal(buf[:, heads:], kept)
