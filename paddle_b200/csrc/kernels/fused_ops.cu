@@ -101,30 +101,35 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 constexpr int RN_THREADS = 256;
 constexpr int RN_MAXIT = 4;
 
-constexpr int RNW_THREADS = 128;   // small CTAs: four rows each, so CTA turnover does not idle half an SM
-// Warp-per-row variant for H = 256 * NV: the row stays in registers as packed bf16 (NV 128-bit words per
-// lane, all loads issued before the first use), the reduction is shuffle-only, no CTA barrier.  With a
-// residual the bf16-rounded sum is what gets normalised (and stored when residual_out is given).
+constexpr int RNW_THREADS = 128;   // small CTAs, so that their turnover does not idle half an SM
+// Few warps per row for H = 256 * NV: the row stays in registers as packed bf16, all loads are issued before the first use, one
+// barrier.  With a residual the bf16-rounded sum is what gets normalised (and stored when residual_out is given).
+// A warp for each row needed 128 registers, 16 rows an SM ran at a time and 4096 rows took 1.7 rounds.  us, one warp / two / four a row:
+// 4096 x 4096 19.1 / 14.7 / 14.7, with residual 37.0 / 27.0 / 24.8, 16384 x 4096 with residual 119 / 86 / 84 (82 at the copy rate), 2331
+// x 5120 14.6 / 12.6 / 12.6, 8192 x 2048 16.7 / 14.6 / 16.6.
+constexpr int rnw_warps(int nv) { return nv <= 8 ? 2 : 4; }
 template <typename WT, int NV>
-__global__ void __launch_bounds__(RNW_THREADS, (NV <= 16 ? 4 : 2)) rms_norm_fwd_warp_kernel(
+__global__ void __launch_bounds__(RNW_THREADS) rms_norm_fwd_warp_kernel(
     const bf16* __restrict__ x, const bf16* __restrict__ residual, const WT* __restrict__ w,
     bf16* __restrict__ y, bf16* __restrict__ residual_out, float* __restrict__ inv_rms, int64_t rows,
     float eps) {
-  constexpr int H = NV * 256;
+  constexpr int H = NV * 256, WPR = rnw_warps(NV), TPR = 32 * WPR, NL = NV / WPR, RPC = RNW_THREADS / TPR;
+  static_assert(NV % WPR == 0, "whole vectors for each warp");
+  __shared__ float red[RNW_THREADS / 32];
   pdl_wait();
   pdl_trigger();
-  const int lane = threadIdx.x & 31;
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * (RNW_THREADS / 32) + (threadIdx.x >> 5);
-  if (row >= rows) return;
+  const int lane = threadIdx.x % TPR;
+  const int64_t my_row = static_cast<int64_t>(blockIdx.x) * RPC + threadIdx.x / TPR, row = min(my_row, rows - 1);
+  const bool live = my_row < rows;                   // the last block may have rows to spare: they read the last one and store nothing
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
-  uint4 cache[NV];
+  uint4 cache[NL];
 #pragma unroll
-  for (int k = 0; k < NV; ++k) cache[k] = __ldg(xr + lane + 32 * k);
+  for (int k = 0; k < NL; ++k) cache[k] = __ldg(xr + lane + TPR * k);
   if (residual != nullptr) {
     const uint4* rr = reinterpret_cast<const uint4*>(residual + row * H);
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      const uint4 rc = __ldg(rr + lane + 32 * k);
+    for (int k = 0; k < NL; ++k) {
+      const uint4 rc = __ldg(rr + lane + TPR * k);
       __nv_bfloat162* a = reinterpret_cast<__nv_bfloat162*>(&cache[k]);
       const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&rc);
 #pragma unroll
@@ -132,13 +137,13 @@ __global__ void __launch_bounds__(RNW_THREADS, (NV <= 16 ? 4 : 2)) rms_norm_fwd_
         const float2 fa = __bfloat1622float2(a[j]), fb = __bfloat1622float2(b[j]);
         a[j] = __floats2bfloat162_rn(fa.x + fb.x, fa.y + fb.y);
       }
-      if (residual_out != nullptr)
-        reinterpret_cast<uint4*>(residual_out + row * H)[lane + 32 * k] = cache[k];
+      if (residual_out != nullptr && live)
+        reinterpret_cast<uint4*>(residual_out + row * H)[lane + TPR * k] = cache[k];
     }
   }
   float ss = 0.f;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
+  for (int k = 0; k < NL; ++k) {
     const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&cache[k]);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -147,10 +152,16 @@ __global__ void __launch_bounds__(RNW_THREADS, (NV <= 16 ? 4 : 2)) rms_norm_fwd_
     }
   }
   ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (!live) return;
+  ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < WPR; ++i) ss += red[threadIdx.x / TPR * WPR + i];
   const float r = rsqrtf(ss / static_cast<float>(H) + eps);
   if (lane == 0 && inv_rms != nullptr) inv_rms[row] = r;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
+  for (int k = 0; k < NL; ++k) {
     float xv[8], wv[8], o[8];
     const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&cache[k]);
 #pragma unroll
@@ -159,10 +170,10 @@ __global__ void __launch_bounds__(RNW_THREADS, (NV <= 16 ? 4 : 2)) rms_norm_fwd_
       xv[2 * j] = f.x;
       xv[2 * j + 1] = f.y;
     }
-    load8(w + (lane + 32 * k) * 8, wv);
+    load8(w + (lane + TPR * k) * 8, wv);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = xv[j] * r * wv[j];
-    store8(y + row * H + (lane + 32 * k) * 8, o);
+    store8(y + row * H + (lane + TPR * k) * 8, o);
   }
 }
 
@@ -892,10 +903,10 @@ PD_EXPORT int pd_rms_norm_fwd(const void* x, const void* residual, const void* w
   if (H % 8 != 0 || rows <= 0) return kErrBadShape;
   const bool al = aligned16(x) && aligned16(y) && aligned16(w) && (residual == nullptr || aligned16(residual)) &&
                   (residual_out == nullptr || aligned16(residual_out));
-  // a warp per row needs rows to fill the GPU; below two per SM a CTA per row is quicker
+  // few warps per row need rows to fill the GPU; below two per SM a larger CTA per row is quicker
 #define PD_RMS_WARP(NV)                                                                                  \
   if (al && H == (NV) * 256 && rows > 2 * sm_count()) {                                                  \
-    const unsigned blocks = static_cast<unsigned>((rows + RNW_THREADS / 32 - 1) / (RNW_THREADS / 32));   \
+    const unsigned blocks = static_cast<unsigned>((rows + RNW_THREADS / 32 / rnw_warps(NV) - 1) / (RNW_THREADS / 32 / rnw_warps(NV)));   \
     return w_is_f32 ? launch_pdl(rms_norm_fwd_warp_kernel<float, NV>, dim3(blocks), dim3(RNW_THREADS), 0, stream, 1,            \
                                  (const bf16*)x, (const bf16*)residual, (const float*)w, (bf16*)y, (bf16*)residual_out, inv_rms, rows, eps) \
                     : launch_pdl(rms_norm_fwd_warp_kernel<bf16, NV>, dim3(blocks), dim3(RNW_THREADS), 0, stream, 1,             \

@@ -331,3 +331,24 @@ def test_rope_whole_blocks_and_teams(tokens, heads, D):
     native.rope(x.unsqueeze(0), cos, sin, out=x.unsqueeze(0), backward=True)
     _lib.check_status()
     assert torch.equal(x, y) and torch.equal(buf[:, heads:], kept)
+
+
+@pytest.mark.parametrize("rows,H", [(297, 2048), (298, 2048), (297, 4096), (301, 5120), (297, 256 * 16)])
+@pytest.mark.parametrize("with_residual", [False, True])
+@pytest.mark.parametrize("wdtype", [torch.bfloat16, torch.float32])
+def test_rms_norm_rows_of_few_warps(rows, H, with_residual, wdtype):
+    """Row lengths that two or four warps share, just above the rows from which they are taken, the last block half empty."""
+    from paddle_b200.ops import _lib, native
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    x, r = (torch.randn(rows, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).to(wdtype)
+    y, inv, out = native.rms_norm_fwd(x, w, 1e-5, r if with_residual else None, with_residual)
+    _lib.check_status()
+    s = (x.float() + r.float()).bfloat16() if with_residual else x
+    if with_residual:
+        assert torch.equal(out, s)
+    d = s.double()
+    ri = torch.rsqrt(d.pow(2).mean(-1) + 1e-5)
+    assert ((inv.double() - ri).abs() <= 1e-5 * ri).all()            # fp32 sums of H squares
+    ref = d * ri[:, None] * w.double()
+    assert ((y.double() - ref).abs() <= (2 ** -8 + 2e-5) * ref.abs()).all()
