@@ -1002,7 +1002,10 @@ PD_EXPORT int pd_swiglu_fwd(const void* x, const void* y, void* out, int64_t row
 PD_EXPORT int pd_swiglu_bwd(const void* x, const void* y, const void* dout, void* dx, void* dy,
                             int64_t rows, int F, int64_t ld_in, cudaStream_t stream) {
   if (F % 8 != 0 || ld_in % 8 != 0 || rows <= 0) return kErrBadShape;
-  swiglu_bwd_kernel<<<grid_for(rows * (F >> 3), 256), 256, 0, stream>>>(
+  // a thread for each vector: blocks that walk on keep five rows a step apart in flight (4096 x 11008 75.4 / 70.0, 8192 x 4096 56.7 /
+  // 53.6 us; the forward kernel, with three, is quicker the other way: 45.2 / 47.3)
+  const int64_t blocks = min((rows * (F >> 3) + 255) / 256, static_cast<int64_t>(INT32_MAX));
+  swiglu_bwd_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
       (const bf16*)x, (const bf16*)y, (const bf16*)dout, (bf16*)dx, (bf16*)dy, rows, F, ld_in);
   return PD_CHECK_LAUNCH();
 }
