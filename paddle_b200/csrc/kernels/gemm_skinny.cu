@@ -20,7 +20,6 @@
 // with split-K atomics and a finalising kernel each: 123 us).  Two 7B layers and the head for one sequence, 1.07 GB of weights
 // (161 us at the copy rate): 382 -> 262 us, with the qkv epilogue, dependent launches and a CTA per row in the norms 216 us;
 // two 13B layers and the head, batch 64, 842 -> 760 -> 717 us (attention 387 of it, at the copy rate).
-// Weights that leave the L2 first and cuts of K into eight for few rows: 215 -> 212 and 712 -> 707 us.
 #include "host_utils.h"
 #include "sm100_prims.cuh"
 
@@ -311,11 +310,12 @@ static int setup(const void* x, const void* w, int M, int N, int K, int ldx, int
     return kErrTensorMap;
   const int kb = (K + BK - 1) / BK;
   if (splits == 0) {
-    // two CTAs per SM in one wave, no CTA with fewer than four blocks of K; from nine rows on at most 4: with 8 the partial tiles
-    // cost more than the further loads in flight bring (us with 4 / 8: K = N = 4096, M = 1 8.7 / 7.7, 128 14.0 / 20.7; K = 11008,
-    // N = 4096, M = 1 16.9 / 15.8, 32 18.9 / 19.5)
+    // two CTAs per SM in one wave, no CTA with fewer than four blocks of K; at most 4: with 8 the partial tiles cost more than the
+    // further loads in flight bring (us with 4 / 8: K = N = 4096, M = 128 14.0 / 20.7; K = 11008, N = 4096, M = 32 18.9 / 19.5).  One row
+    // would gain (8.7 / 7.7 and 16.9 / 15.8), but the number of cuts is the order in which a row is summed up: it must not follow M, or
+    // a sequence's result changes with the number of those that are decoded beside it.
     splits = 1;
-    while (splits < (M <= 8 ? MAX_SPLIT : 4) && tiles * splits * 2 <= 2 * sm_count() && kb >= 8 * splits) splits *= 2;
+    while (splits < 4 && tiles * splits * 2 <= 2 * sm_count() && kb >= 8 * splits) splits *= 2;
   }
   p->M = M;
   p->N = N;

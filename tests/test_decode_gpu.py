@@ -123,6 +123,23 @@ def test_skinny_gemm(M, K_, N, splits):
         assert (got.double() - ref).abs().le(ref.abs() * 2 ** -8 + 1e-4).all()
 
 
+@pytest.mark.parametrize("K_,N", [(4096, 136), (4096, 4096), (11008, 4096)])
+def test_skinny_rows_do_not_depend_on_the_batch(K_, N):
+    """A row is summed up in the same order whatever the number of rows: by default in as many cuts of K for one row as for nine or
+    more, at most four."""
+    from paddle_b200.ops import native, _lib
+    g = torch.Generator(device="cuda").manual_seed(K_ + N)
+    x = torch.randn(65, K_, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(K_, N, device="cuda", generator=g) * 0.05).bfloat16()
+    one = native.gemm_skinny(x[:1], w)
+    for M in (2, 8, 9, 16, 17, 33, 65):
+        assert torch.equal(native.gemm_skinny(x[:M], w)[:1], one), M
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert torch.equal(native.gemm_skinny(x[:1], w, splits=4), one)
+    torch.cuda.synchronize()
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("M,H,N", [(1, 512, 1536), (17, 2048, 5120), (128, 4096, 1024)])
 def test_skinny_gemm_behind_the_kernels_of_a_decode_step(M, H, N):
     """As a decode step launches it, with weights fetched ahead of the wait: the norm kernel just before writes x and the residual,
