@@ -158,7 +158,7 @@ struct Operands {
 template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int N, int mn3d, int splits, int* status,
-                  const __nv_bfloat16* bias, int act, const __nv_bfloat16* residual, int ldr) {
+                  const __nv_bfloat16* bias, int act, const __nv_bfloat16* residual, int ldr, int round_product) {
   // accumulators hold ACC_N columns; a 512-column tile takes both of one tile, narrower ones alternate between tiles
   constexpr int ACC_N = TILE_N == 512 ? 256 : TILE_N, HALVES = TILE_N / ACC_N;
   constexpr int STAGES = stages(TILE_N), BN_HALF = ACC_N / 2, B_STAGE_BYTES = b_stage_bytes(TILE_N), B_HALF_BYTES = B_STAGE_BYTES / HALVES;
@@ -430,7 +430,8 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
                 for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(apply_act(__uint_as_float(r[i]), act));
               }
               // a residual added by a kernel of its own moves the product through memory twice more: a prompt of 3 x 777 tokens
-              // through one 13B layer 1507 -> 1481 us, two additions of 14 each
+              // through one 13B layer 1507 -> 1481 us, two additions of 14 each.  With
+              // round_product the addition starts from what that kernel is given, a product in bf16.
               if (residual != nullptr && m0 + epi_tid < M) {      // N % 8 == 0: a group of eight columns is inside or outside
                 const __nv_bfloat16* rp = residual + static_cast<int64_t>(m0 + epi_tid) * ldr + col0;
 #pragma unroll
@@ -440,8 +441,13 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
                     const uint32_t w[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                      r[8 * q + 2 * e] = __float_as_uint(__uint_as_float(r[8 * q + 2 * e]) + __uint_as_float(w[e] << 16));
-                      r[8 * q + 2 * e + 1] = __float_as_uint(__uint_as_float(r[8 * q + 2 * e + 1]) + __uint_as_float(w[e] & 0xffff0000u));
+                      float y0 = __uint_as_float(r[8 * q + 2 * e]), y1 = __uint_as_float(r[8 * q + 2 * e + 1]);
+                      if (round_product) {
+                        const uint32_t y = pack_bf16x2(y0, y1);
+                        y0 = __uint_as_float(y << 16), y1 = __uint_as_float(y & 0xffff0000u);
+                      }
+                      r[8 * q + 2 * e] = __float_as_uint(y0 + __uint_as_float(w[e] << 16));
+                      r[8 * q + 2 * e + 1] = __float_as_uint(y1 + __uint_as_float(w[e] & 0xffff0000u));
                     }
                   }
                 }
@@ -505,7 +511,7 @@ static int max_clusters(int max_ctas) {
 template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G = 1>
 static int launch_variant(const Operands<G>& op, int groups, int M, int N, int mn3d, int* status, cudaStream_t stream, int max_ctas,
                           int splits, const __nv_bfloat16* bias = nullptr, int act = 0, const __nv_bfloat16* residual = nullptr,
-                          int ldr = 0) {
+                          int ldr = 0, int round_product = 0) {
   auto kfn = gemm2_bf16_kernel<A_MN, B_MN, EPI, TILE_N, G>;
   static bool configured = false;
   if (!configured) {
@@ -515,7 +521,8 @@ static int launch_variant(const Operands<G>& op, int groups, int M, int N, int m
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N) * splits * groups;
   int clusters = max_clusters(max_ctas);
   if (clusters > tiles) clusters = tiles;
-  kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(op, groups, M, N, mn3d, splits, status, bias, act, residual, ldr);
+  kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(op, groups, M, N, mn3d, splits, status, bias, act, residual, ldr,
+                                                                round_product);
   return cudaGetLastError() == cudaSuccess ? kLaunchOk : kErrCuda;
 }
 
@@ -583,11 +590,11 @@ PD_EXPORT int pd_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, in
 }
 
 // C = act(A B + bias) + residual (swiglu = 0; C bf16 [M, N]; bias and residual may be null; with a residual N and ldr are multiples of
-// 8) or C = silu(gate) * up over interleaved (gate, up) column pairs (swiglu = 1; C bf16 [M, N / 2], N a multiple of 16, bias and
-// residual must be null).  Operand layouts as pd_gemm_bf16_2cta.
+// 8; round_product = 1: what it is added to is rounded to bf16 first) or C = silu(gate) * up over interleaved (gate, up) column pairs
+// (swiglu = 1; C bf16 [M, N / 2], N a multiple of 16, bias and residual must be null).  Operand layouts as pd_gemm_bf16_2cta.
 PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                                     int a_mn_major, int b_mn_major, const void* bias, int act, int swiglu, const void* residual, int ldr,
-                                    int* status, cudaStream_t stream) {
+                                    int round_product, int* status, cudaStream_t stream) {
   using namespace pd;
   using namespace pd::gemm2;
   if (M <= 0 || N <= 0 || K <= 0 || act < 0 || act > 4) return kErrBadShape;
@@ -609,9 +616,9 @@ PD_EXPORT int pd_gemm_bf16_2cta_epi(const void* A, const void* B, void* C, int M
 #define PD_GEMM2_EPI_CASE(AM, BM_)                                                                              \
   if (a_mn_major == AM && b_mn_major == BM_) {                                                                  \
     if (swiglu) return launch_variant<AM, BM_, kSwiglu, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1); \
-    return TN == 512 ? launch_variant<AM, BM_, kBiasAct, 512>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr) \
-         : TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr) \
-                     : launch_variant<AM, BM_, kBiasAct, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr); \
+    return TN == 512 ? launch_variant<AM, BM_, kBiasAct, 512>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr, round_product) \
+         : TN == 128 ? launch_variant<AM, BM_, kBiasAct, 128>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr, round_product) \
+                     : launch_variant<AM, BM_, kBiasAct, 256>(op, 1, M, N, a3d | (b3d << 1), status, stream, 0, 1, bp, act, rp, ldr, round_product); \
   }
   PD_GEMM2_EPI_CASE(0, 0) PD_GEMM2_EPI_CASE(0, 1) PD_GEMM2_EPI_CASE(1, 0) PD_GEMM2_EPI_CASE(1, 1)
 #undef PD_GEMM2_EPI_CASE

@@ -283,7 +283,7 @@ class FusedMultiTransformer(Layer):
         if residual is None:
             return native.gemm(x, w)
         if native.GEMM_IMPL == "2cta" and w.shape[1] % 8 == 0 and native.rows16(residual):
-            return native.gemm_epilogue(x, w, residual=residual)
+            return native.gemm_epilogue(x, w, residual=residual, round_product=True)
         y = native.gemm(x, w)
         return native.add_bf16(y, residual, out=y)
 

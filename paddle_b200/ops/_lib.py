@@ -54,7 +54,7 @@ def _load(name: str, builder: str):
 # them declared, ctypes converts plain numbers and addresses itself: a call of 16 arguments costs 3 us less than one that
 # wraps each in a ctypes object.
 _SIGNATURES = {
-    "pd_gemm_bf16_2cta": "ppp iiiiiiiiiii pp", "pd_gemm_bf16_2cta_epi": "ppp iiiiiiii p ii pi pp",
+    "pd_gemm_bf16_2cta": "ppp iiiiiiiiiii pp", "pd_gemm_bf16_2cta_epi": "ppp iiiiiiii p ii pii pp",
     "pd_gemm_skinny": "ppp iiiiii pp iiii pp", "pd_gemm_bf16_grouped_tn": "ppppp iiiiii l i pp",
     "pd_rms_norm_fwd": "ppp i ppp l i f p", "pd_rms_norm_bwd": "ppp i ppppp i l i p", "pd_rms_norm_bwd_parts": "l",
     "pd_rope": "ppppp l ii ll iii p", "pd_swiglu_fwd": "ppp l i l p", "pd_swiglu_bwd": "ppppp l i l p",

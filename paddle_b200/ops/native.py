@@ -474,10 +474,11 @@ ACT_CODES = {None: 0, "none": 0, "identity": 0, "relu": 1, "gelu": 2, "gelu_tanh
 
 
 @plain_dispatch
-def gemm_epilogue(a, b, bias=None, act=None, trans_a=False, trans_b=False, swiglu=False, out=None, residual=None):
+def gemm_epilogue(a, b, bias=None, act=None, trans_a=False, trans_b=False, swiglu=False, out=None, residual=None, round_product=False):
     """``act(op(a) @ op(b) + bias) + residual`` in one kernel (bias bf16 ``[N]``, residual bf16 ``[M, N]``; act in ``ACT_CODES``),
     or with ``swiglu=True`` ``silu(gate) * up`` over the interleaved (gate, up) column pairs of the product, returning
-    ``[M, N / 2]``."""
+    ``[M, N / 2]``.  ``round_product`` rounds the value to bf16 before the residual is added, as :func:`add_bf16` on the
+    result does."""
     _req(a.dtype == BF16 and b.dtype == BF16 and a.dim() == 2 and b.dim() == 2, "gemm_epilogue: 2-D bf16 operands required")
     _req(a.stride(1) == 1 and b.stride(1) == 1, "gemm_epilogue: operands need a unit inner stride")
     M, K = (a.shape[1], a.shape[0]) if trans_a else (a.shape[0], a.shape[1])
@@ -494,13 +495,14 @@ def gemm_epilogue(a, b, bias=None, act=None, trans_a=False, trans_b=False, swigl
     _req(out.dtype == BF16 and tuple(out.shape) == (M, n_out) and out.stride(1) == 1, "gemm_epilogue: bad `out`")
     _req(residual is None or (residual.dtype == BF16 and tuple(residual.shape) == (M, N) and residual.stride(1) == 1),
          "gemm_epilogue: bad residual")
-    if M <= SKINNY_ROWS and ACT_CODES[act] == 0 and not (swiglu or trans_a or trans_b) and gemm_skinny_ok(a, b) and rows16(out) \
-            and (bias is None or bias.data_ptr() % 16 == 0) and (residual is None or rows16(residual)):
+    if M <= SKINNY_ROWS and ACT_CODES[act] == 0 and not (swiglu or trans_a or trans_b or round_product) \
+            and gemm_skinny_ok(a, b) and rows16(out) and (bias is None or bias.data_ptr() % 16 == 0) and (residual is None or rows16(residual)):
         return gemm_skinny(a, b, bias=bias, residual=residual, out=out)
     rc = _lib.kernels().pd_gemm_bf16_2cta_epi(
         addr(a), addr(b), addr(out), M, N, K, a.stride(0), b.stride(0),
         out.stride(0), 1 if trans_a else 0, 0 if trans_b else 1, addr(bias), ACT_CODES[act],
-        1 if swiglu else 0, addr(residual), 0 if residual is None else residual.stride(0), addr(_lib.status_buffer(a.device)), raw_stream())
+        1 if swiglu else 0, addr(residual), 0 if residual is None else residual.stride(0),
+        1 if round_product else 0, addr(_lib.status_buffer(a.device)), raw_stream())
     check(rc, "pd_gemm_bf16_2cta_epi")
     _count()
     return out

@@ -352,3 +352,18 @@ def test_rms_norm_rows_of_few_warps(rows, H, with_residual, wdtype):
     assert ((inv.double() - ri).abs() <= 1e-5 * ri).all()            # fp32 sums of H squares
     ref = d * ri[:, None] * w.double()
     assert ((y.double() - ref).abs() <= (2 ** -8 + 2e-5) * ref.abs()).all()
+
+
+@pytest.mark.parametrize("M,N,K,width", [(129, 264, 200, 128), (2331, 5120, 512, 256), (2048, 2600, 8200, 512), (2048, 2840, 8200, 512)])
+def test_projection_adds_the_residual_to_a_bf16_product(M, N, K, width):
+    """The projections of prompt processing: the product in bf16, then the residual, in one kernel with every width of its tiles."""
+    from types import SimpleNamespace
+    from paddle_b200.incubate.nn import FusedMultiTransformer
+    from paddle_b200.ops import _lib, native
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _lib.kernels().pd_gemm_2cta_tile_n_at(M, N, K, 1, 0) == width
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w, res = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((M, K), (K, N), (M, N)))
+    got = FusedMultiTransformer._gemm(SimpleNamespace(_ws={"out": (1, None)}), "out", x, w, residual=res)
+    _lib.check_status()
+    assert torch.equal(got, native.add_bf16(native.gemm(x, w), res))
