@@ -102,34 +102,38 @@ constexpr int RN_THREADS = 256;
 constexpr int RN_MAXIT = 4;
 
 constexpr int RNW_THREADS = 128;   // small CTAs, so that their turnover does not idle half an SM
-// Few warps per row for H = 256 * NV: the row stays in registers as packed bf16, all loads are issued before the first use, one
-// barrier.  With a residual the bf16-rounded sum is what gets normalised (and stored when residual_out is given).
-// A warp for each row needed 128 registers, 16 rows an SM ran at a time and 4096 rows took 1.7 rounds.  us, one warp / two / four a row:
-// 4096 x 4096 19.1 / 14.7 / 14.7, with residual 37.0 / 27.0 / 24.8, 16384 x 4096 with residual 119 / 86 / 84 (82 at the copy rate), 2331
-// x 5120 14.6 / 12.6 / 12.6, 8192 x 2048 16.7 / 14.6 / 16.6.
+// Few warps per row for H = 256 * NV: the row stays in registers as packed bf16 and all loads are issued before the first use.  With a
+// residual the bf16-rounded sum is what gets normalised (and stored when residual_out is given).
+// Lane l adds up the vectors l, l + 32, l + 64, ... of a row one after the other and the lanes are added at the end, whatever the number
+// of warps: a warp holds consecutive groups of 32 vectors and goes on from the sums of the warp before it.
+// A warp for each row needed 128 registers: 16 warps an SM, each a chain of loads, sums and stores of a whole row; now some 32 are
+// active, with shorter chains.  us, one warp a row / this: 4096 x 4096 18.9 / 14.8, with residual 37.0 / 24.9, 16384 x 4096 with
+// residual 119 / 84 (82 at the copy rate), 2331 x 5120 14.5 / 12.5, 8192 x 2048 16.7 / 14.6; two warps for 4096 and 5120 16.6, 33.1,
+// 103, 14.5.
 constexpr int rnw_warps(int nv) { return nv <= 8 ? 2 : 4; }
-template <typename WT, int NV>
-__global__ void __launch_bounds__(RNW_THREADS) rms_norm_fwd_warp_kernel(
+template <typename WT, int NV, bool RES>
+__global__ void __launch_bounds__(RNW_THREADS) rms_norm_fwd_rows_kernel(
     const bf16* __restrict__ x, const bf16* __restrict__ residual, const WT* __restrict__ w,
     bf16* __restrict__ y, bf16* __restrict__ residual_out, float* __restrict__ inv_rms, int64_t rows,
     float eps) {
   constexpr int H = NV * 256, WPR = rnw_warps(NV), TPR = 32 * WPR, NL = NV / WPR, RPC = RNW_THREADS / TPR;
   static_assert(NV % WPR == 0, "whole vectors for each warp");
-  __shared__ float red[RNW_THREADS / 32];
+  __shared__ float red[RPC][32];
   pdl_wait();
   pdl_trigger();
-  const int lane = threadIdx.x % TPR;
-  const int64_t my_row = static_cast<int64_t>(blockIdx.x) * RPC + threadIdx.x / TPR, row = min(my_row, rows - 1);
+  const int team = threadIdx.x / TPR, warp = threadIdx.x % TPR >> 5, lane = threadIdx.x & 31;
+  const int first = lane + 32 * NL * warp;           // of the vectors of this thread, 32 apart
+  const int64_t my_row = static_cast<int64_t>(blockIdx.x) * RPC + team, row = min(my_row, rows - 1);
   const bool live = my_row < rows;                   // the last block may have rows to spare: they read the last one and store nothing
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
   uint4 cache[NL];
 #pragma unroll
-  for (int k = 0; k < NL; ++k) cache[k] = __ldg(xr + lane + TPR * k);
-  if (residual != nullptr) {
+  for (int k = 0; k < NL; ++k) cache[k] = __ldg(xr + first + 32 * k);
+  if (RES) {
     const uint4* rr = reinterpret_cast<const uint4*>(residual + row * H);
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
-      const uint4 rc = __ldg(rr + lane + TPR * k);
+      const uint4 rc = __ldg(rr + first + 32 * k);
       __nv_bfloat162* a = reinterpret_cast<__nv_bfloat162*>(&cache[k]);
       const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&rc);
 #pragma unroll
@@ -138,28 +142,34 @@ __global__ void __launch_bounds__(RNW_THREADS) rms_norm_fwd_warp_kernel(
         a[j] = __floats2bfloat162_rn(fa.x + fb.x, fa.y + fb.y);
       }
       if (residual_out != nullptr && live)
-        reinterpret_cast<uint4*>(residual_out + row * H)[lane + TPR * k] = cache[k];
+        reinterpret_cast<uint4*>(residual_out + row * H)[first + 32 * k] = cache[k];
     }
   }
-  float ss = 0.f;
+  // with a residual the squares are made before their turn, without one in it (us, before / in: 4096 x 4096 16.8 / 14.8, with residual
+  // 24.9 / 28.8)
+  float sq[4 * NL];
+  auto square = [&](int k, int j) {
+    const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&cache[k])[j]);
+    return f.x * f.x + f.y * f.y;
+  };
+  if (RES) {
 #pragma unroll
-  for (int k = 0; k < NL; ++k) {
-    const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&cache[k]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __bfloat1622float2(a[j]);
-      ss += f.x * f.x + f.y * f.y;
-    }
+    for (int k = 0; k < 4 * NL; ++k) sq[k] = square(k >> 2, k & 3);
   }
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < WPR; ++i) {
+    if (warp == i) {
+      float s = i == 0 ? 0.f : red[team][lane];
+#pragma unroll
+      for (int k = 0; k < 4 * NL; ++k) s += RES ? sq[k] : square(k >> 2, k & 3);
+      red[team][lane] = s;
+    }
+    __syncthreads();
+  }
   if (!live) return;
-  ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < WPR; ++i) ss += red[threadIdx.x / TPR * WPR + i];
+  const float ss = warp_sum(red[team][lane]);
   const float r = rsqrtf(ss / static_cast<float>(H) + eps);
-  if (lane == 0 && inv_rms != nullptr) inv_rms[row] = r;
+  if (first == 0 && inv_rms != nullptr) inv_rms[row] = r;
 #pragma unroll
   for (int k = 0; k < NL; ++k) {
     float xv[8], wv[8], o[8];
@@ -170,10 +180,10 @@ __global__ void __launch_bounds__(RNW_THREADS) rms_norm_fwd_warp_kernel(
       xv[2 * j] = f.x;
       xv[2 * j + 1] = f.y;
     }
-    load8(w + (lane + TPR * k) * 8, wv);
+    load8(w + (first + 32 * k) * 8, wv);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = xv[j] * r * wv[j];
-    store8(y + row * H + (lane + TPR * k) * 8, o);
+    store8(y + row * H + (first + 32 * k) * 8, o);
   }
 }
 
@@ -904,18 +914,21 @@ PD_EXPORT int pd_rms_norm_fwd(const void* x, const void* residual, const void* w
   const bool al = aligned16(x) && aligned16(y) && aligned16(w) && (residual == nullptr || aligned16(residual)) &&
                   (residual_out == nullptr || aligned16(residual_out));
   // few warps per row need rows to fill the GPU; below two per SM a larger CTA per row is quicker
-#define PD_RMS_WARP(NV)                                                                                  \
-  if (al && H == (NV) * 256 && rows > 2 * sm_count()) {                                                  \
-    const unsigned blocks = static_cast<unsigned>((rows + RNW_THREADS / 32 / rnw_warps(NV) - 1) / (RNW_THREADS / 32 / rnw_warps(NV)));   \
-    return w_is_f32 ? launch_pdl(rms_norm_fwd_warp_kernel<float, NV>, dim3(blocks), dim3(RNW_THREADS), 0, stream, 1,            \
-                                 (const bf16*)x, (const bf16*)residual, (const float*)w, (bf16*)y, (bf16*)residual_out, inv_rms, rows, eps) \
-                    : launch_pdl(rms_norm_fwd_warp_kernel<bf16, NV>, dim3(blocks), dim3(RNW_THREADS), 0, stream, 1,             \
-                                 (const bf16*)x, (const bf16*)residual, (const bf16*)w, (bf16*)y, (bf16*)residual_out, inv_rms, rows, eps); \
+#define PD_RMS_ROWS_AS(WT, NV, RES)                                                                          \
+  launch_pdl(rms_norm_fwd_rows_kernel<WT, NV, RES>, dim3(blocks), dim3(RNW_THREADS), 0, stream, 1, (const bf16*)x, (const bf16*)residual, \
+             (const WT*)w, (bf16*)y, (bf16*)residual_out, inv_rms, rows, eps)
+#define PD_RMS_ROWS(NV)                                                                                      \
+  if (al && H == (NV) * 256 && rows > 2 * sm_count()) {                                                      \
+    constexpr int per_block = RNW_THREADS / 32 / rnw_warps(NV);                                              \
+    const unsigned blocks = static_cast<unsigned>((rows + per_block - 1) / per_block);                       \
+    if (residual != nullptr) return w_is_f32 ? PD_RMS_ROWS_AS(float, NV, true) : PD_RMS_ROWS_AS(bf16, NV, true);   \
+    return w_is_f32 ? PD_RMS_ROWS_AS(float, NV, false) : PD_RMS_ROWS_AS(bf16, NV, false);                    \
   }
-  PD_RMS_WARP(8)
-  PD_RMS_WARP(16)
-  PD_RMS_WARP(20)
-#undef PD_RMS_WARP
+  PD_RMS_ROWS(8)
+  PD_RMS_ROWS(16)
+  PD_RMS_ROWS(20)
+#undef PD_RMS_ROWS
+#undef PD_RMS_ROWS_AS
   return w_is_f32 ? launch_pdl(rms_norm_fwd_kernel<float>, dim3(static_cast<unsigned>(rows)), dim3(RN_THREADS), 0, stream, 1, (const bf16*)x,
                                (const bf16*)residual, (const float*)w, (bf16*)y, (bf16*)residual_out, inv_rms, H, eps)
                   : launch_pdl(rms_norm_fwd_kernel<bf16>, dim3(static_cast<unsigned>(rows)), dim3(RN_THREADS), 0, stream, 1, (const bf16*)x,

@@ -367,3 +367,30 @@ def test_projection_adds_the_residual_to_a_bf16_product(M, N, K, width):
     got = FusedMultiTransformer._gemm(SimpleNamespace(_ws={"out": (1, None)}), "out", x, w, residual=res)
     _lib.check_status()
     assert torch.equal(got, native.add_bf16(native.gemm(x, w), res))
+
+
+@pytest.mark.parametrize("rows,H", [(297, 2048), (300, 4096), (299, 5120)])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_rms_norm_rows_are_added_up_lane_by_lane(rows, H, with_residual):
+    """However many warps share a row, lane l adds up the vectors l, l + 32, ... one after the other and the lanes come last.  Rows in
+    which that order shows: a large first element of a lane, which the small ones behind it cannot change."""
+    from paddle_b200.ops import _lib, native
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x = torch.randn(rows, H // 8, 8, device="cuda", generator=g)
+    x[1::2] = 0
+    x[1::2, :, 0::2] = 1.0                    # squares of 1, one in a pair
+    x[1::2, :32, 0] = 2.0 ** 12               # 2^24 + 1 is 2^24 in fp32
+    x = x.reshape(rows, H).bfloat16()
+    inv = native.rms_norm_fwd(x, torch.ones(H, device="cuda"), 1e-5, torch.zeros_like(x) if with_residual else None)[1]
+    _lib.check_status()
+    pairs = x.float().square().reshape(rows, H // 256, 32, 4, 2).sum(-1)       # squares of bf16 are exact, a pair rounds once
+    lanes = torch.zeros(rows, 32, device="cuda")
+    for k in range(H // 256):
+        for j in range(4):
+            lanes = lanes + pairs[:, k, :, j]
+    for o in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[:, torch.arange(32, device="cuda") ^ o]
+    ref = torch.rsqrt(lanes[:, 0].double() / H + 1e-5)
+    # quotient and root in fp32; sums of warps that start from zero keep their H / 512 or more vectors of four ones: 2^-22 or more of the root
+    off = ((inv.double() - ref) / ref).abs()
+    assert off.max() <= 2.5 * 2 ** -23, off.max().item() * 2 ** 23
