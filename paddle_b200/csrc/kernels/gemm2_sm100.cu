@@ -119,11 +119,8 @@ __device__ __forceinline__ void tma2_load_3d(void* smem_dst, const CUtensorMap* 
       : "memory");
 }
 
-__device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
-  // 256-row tiles per raster group: their rows of A stay in the L2 while the columns of B pass once.  Under sustained load (the power
-  // cap), us with 4 / 8 / 16 / 32: 4096 x 12288 x 4096 335 / 316 / 305 / -, its weight gradient 362 / 343 / 331 / -, 2331 x 27648 x
-  // 5120 - / 571 / 540 / 544, 8192 x 4096 x 4096 - / 214 / 210 / 224 (there the group's own rows no longer stay).
-  constexpr int G = 16;
+// Tiles go in groups of G row tiles, column by column.
+__device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int G, int& tm, int& tn) {
   const int per_group = G * tiles_n;
   const int g = t / per_group;
   const int first_m = g * G;
@@ -158,7 +155,7 @@ struct Operands {
 template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int N, int mn3d, int splits, int* status,
-                  const __nv_bfloat16* bias, int act, const __nv_bfloat16* residual, int ldr, int round_product) {
+                  const __nv_bfloat16* bias, int act, const __nv_bfloat16* residual, int ldr, int round_product, int raster) {
   // accumulators hold ACC_N columns; a 512-column tile takes both of one tile, narrower ones alternate between tiles
   constexpr int ACC_N = TILE_N == 512 ? 256 : TILE_N, HALVES = TILE_N / ACC_N;
   constexpr int STAGES = stages(TILE_N), BN_HALF = ACC_N / 2, B_STAGE_BYTES = b_stage_bytes(TILE_N), B_HALF_BYTES = B_STAGE_BYTES / HALVES;
@@ -223,7 +220,7 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters) {
         int tm, tn, kb0, kb1;
         const int g = group_of(t), tg = t - g * group_tiles;
-        tile_coords(tg / splits, tiles_m, tiles_n, tm, tn);
+        tile_coords(tg / splits, tiles_m, tiles_n, raster, tm, tn);
         const int m0 = tm * TILE_M + static_cast<int>(cta_rank) * BM;
         const int n0 = tn * TILE_N + static_cast<int>(cta_rank) * BN_HALF, halves = halves_at(tn * TILE_N);
         k_range(g, tg, kb0, kb1);
@@ -266,7 +263,7 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
         for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {
           const int g = group_of(t), tg = t - g * group_tiles;
           int tm_, tn, kb0, kb1;
-          tile_coords(tg / splits, tiles_m, tiles_n, tm_, tn);
+          tile_coords(tg / splits, tiles_m, tiles_n, raster, tm_, tn);
           k_range(g, tg, kb0, kb1);
           const int halves = halves_at(tn * TILE_N);
           if (!mbar_wait_warp(&bars->tempty[0], (it & 1) ^ 1, abort_flag, status, 200)) { ok = false; break; }
@@ -353,7 +350,7 @@ gemm2_bf16_kernel(const __grid_constant__ Operands<G> op, int groups, int M, int
     for (int t = cluster_id; t < num_tiles && live; t += n_clusters, ++it) {
       int tm, tn;
       const int g = group_of(t);
-      tile_coords((t - g * group_tiles) / splits, tiles_m, tiles_n, tm, tn);
+      tile_coords((t - g * group_tiles) / splits, tiles_m, tiles_n, raster, tm, tn);
       const int m0 = tm * TILE_M + static_cast<int>(cta_rank) * BM;
       const int halves = halves_at(tn * TILE_N);
 #pragma unroll 1
@@ -508,6 +505,17 @@ static int max_clusters(int max_ctas) {
   return clusters < 1 ? 1 : clusters;
 }
 
+// Row tiles of a raster group (tile_coords): their rows of A stay in the L2 while the columns of B pass once.  Sixteen: under sustained
+// load (the power cap), us with 4 / 8 / 16 / 32: 4096 x 12288 x 4096 335 / 316 / 305 / -, its weight gradient 362 / 343 / 331 / -,
+// 2331 x 27648 x 5120 - / 552 / 526 / 544; 8 / 16: 8192 x 12288 x 4096 628 / 603, 8192 x 11008 x 4096 561 / 543, 5120 x 12288 x 4096
+// 397 / 380, 8192 x 5120 x 5120 330 / 330, 16384 x 4096 x 4096 415 / 414.  Thirty-two lose their own rows (8192 x 4096 x 5120 258 / 263 /
+// 289 with 8 / 16 / 32).  Of deep products (K >= 8192) sixteen row tiles of A are 64 MB of the 126 MB and more, so tiles of 256 columns
+// take eight there: 8 / 16, 8192 x 4096 x 8192 445 / 450, x 11008 573 / 582, x 13824 721 / 734, 4096 x 22016 x 8200 1221 / 1250, 4096 x
+// 5120 x 13824 483 / 488, 22016 x 4096 x 16384 into fp32 2510 / 2581; with K = 7168 483 / 487, with 6144 417 / 413.  Up to fifteen row
+// tiles would be cut into two groups: 2331 x 5120 x 13824 301 / 292.  Tiles of 512 columns pass over A half as often: 8192 x 8192 x
+// 11008 1106 / 1086, 4096 x 4096 x 22016 575 / 566.
+static int raster_rows(int tile_n, int M, int K) { return tile_n == 256 && K >= 8192 && M > 15 * TILE_M ? 8 : 16; }
+
 template <bool A_MN, bool B_MN, int EPI, int TILE_N, int G = 1>
 static int launch_variant(const Operands<G>& op, int groups, int M, int N, int mn3d, int* status, cudaStream_t stream, int max_ctas,
                           int splits, const __nv_bfloat16* bias = nullptr, int act = 0, const __nv_bfloat16* residual = nullptr,
@@ -522,7 +530,7 @@ static int launch_variant(const Operands<G>& op, int groups, int M, int N, int m
   int clusters = max_clusters(max_ctas);
   if (clusters > tiles) clusters = tiles;
   kfn<<<clusters * 2, NUM_THREADS, smem_bytes(TILE_N), stream>>>(op, groups, M, N, mn3d, splits, status, bias, act, residual, ldr,
-                                                                round_product);
+                                                                round_product, raster_rows(TILE_N, M, op.k[0]));
   return cudaGetLastError() == cudaSuccess ? kLaunchOk : kErrCuda;
 }
 

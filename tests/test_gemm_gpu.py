@@ -203,3 +203,25 @@ def test_deep_products_take_wide_tiles(M, N, K_, max_ctas, width, ta, tb):
     assert (native.gemm_epilogue(a, b, bias, None, ta, tb).double() - ref - bias.double()).abs().le(tol + bias.double().abs() * 2 ** -8).all()
     torch.cuda.synchronize()
     _lib.check_status()
+
+
+@pytest.mark.parametrize("M,N,K_,width", [(4360, 264, 136, 128), (8200, 520, 136, 256), (4360, 776, 8200, 256), (3848, 776, 8200, 256),
+                                          (3840, 776, 8200, 256), (4360, 1304, 8200, 512)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, True)])
+def test_row_tiles_of_several_raster_groups(M, N, K_, width, ta, tb):
+    """More row tiles than a raster group holds, the last group ragged: 18 and 33 in groups of 16, deep ones with 256 columns in groups
+    of 8 from 16 row tiles on, in one group of 16 with 15."""
+    from paddle_b200.ops import _lib, native
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _lib.kernels().pd_gemm_2cta_tile_n_at(M, N, K_, 1, 0) == width
+    a, b = _mk(M, N, K_, ta, tb)
+    ref = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    # as test_deep_products_take_wide_tiles: K_ / 16 steps lose up to 2^-23 of a running sum below 5 sqrt(K_); one rounding to bf16
+    sums = K_ / 16 * 5 * K_ ** 0.5 * 2 ** -23 + 1e-5
+    got = native.gemm(a, b, ta, tb)
+    _lib.check_status()
+    assert (got.double() - ref).abs().le(ref.abs() * 2 ** -8 + sums).all()
+    acc = torch.ones(M, N, device="cuda")
+    native.gemm(a, b, ta, tb, out=acc, accumulate=True)
+    _lib.check_status()
+    assert (acc.double() - 1 - ref).abs().max() <= sums + 1e-4
