@@ -97,6 +97,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                  const __grid_constant__ CUtensorMap tmDK,
                  const __grid_constant__ CUtensorMap tmDV, Params p, int head_chunk) {
+  pdl_wait();                                        // Delta and the cleared dQ sums, should this ever start under the kernel that makes them
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
@@ -142,7 +143,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int n_it = per_head * group;
 
   if (threadIdx.x == 0) {
-    pdl_trigger();                                   // the conversion of dQ: waits for this kernel before it reads anything
+    pdl_trigger();                                   // after pdl_wait above; the conversion of dQ waits for this kernel before it reads
     mbar_init(&bars->kv_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&bars->qdo_full[s], 1);

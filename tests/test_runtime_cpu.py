@@ -139,3 +139,30 @@ def test_runtime_under_sanitizer(sanitizer):
                        env=env, cwd=root, capture_output=True, text=True, timeout=600)
     report = [l for l in (p.stdout + p.stderr).splitlines() if "Sanitizer" in l and ("ERROR" in l or "WARNING" in l)]
     assert p.returncode == 0 and not report, (p.stdout[-1500:], p.stderr[-1500:])
+
+
+def test_early_starting_kernels_wait_before_they_trigger():
+    """The rule of programmatic dependent launches (sm100_prims.cuh): a kernel that lets its successor start has waited for its
+    predecessor, and a kernel launched with launch_pdl waits.  Read from the sources: body by body of the __global__ functions."""
+    import glob
+    import os
+    import re
+    import paddle_b200
+    kernels, launched = {}, set()
+    for path in glob.glob(os.path.join(os.path.dirname(paddle_b200.__file__), "csrc", "kernels", "*.cu")):
+        src = re.sub(r"//[^\n]*", "", open(path).read())
+        names = re.findall(r"launch_pdl\(\s*(\w+)", src)
+        launched |= {m for v in names for m in [v] + re.findall(r"auto\s+%s\s*=\s*(\w+)" % v, src)}
+        src = re.sub(r"__launch_bounds__\([^)]*(\([^)]*\)[^)]*)*\)|__cluster_dims__\([^)]*\)", "", src)
+        for part in src.split("__global__")[1:]:
+            body = part[part.index("{"):]
+            kernels.setdefault(re.search(r"(\w+)\s*\(", part).group(1), []).append(body[:body.index("\n}")])
+    with_trigger = [n for n, bodies in kernels.items() if any("pdl_trigger(" in b for b in bodies)]
+    assert len(with_trigger) >= 4
+    for n in with_trigger:
+        for b in kernels[n]:
+            t = b.find("pdl_trigger(")
+            assert t < 0 or 0 <= b.find("pdl_wait(") < t, n
+    for n in launched & set(kernels):
+        assert all("pdl_wait(" in b for b in kernels[n]), n
+    assert {"dq_convert_kernel", "skinny_gemm_kernel", "rms_norm_fwd_rows_kernel"} <= launched & set(kernels)
