@@ -140,6 +140,33 @@ def test_skinny_rows_do_not_depend_on_the_batch(K_, N):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("M", [1, 33])
+@pytest.mark.parametrize("N", [9208, 9216, 9232])
+def test_skinny_gemm_of_weights_that_leave_the_l2_first(M, N):
+    """Weights just below 72 MB, of 72 MB and above, from where on they are loaded with an L2 policy: bias and residual, and the two
+    column halves of the activation, with weights fetched ahead of the wait."""
+    from paddle_b200.ops import native, _lib
+    K_ = 4096
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = (torch.randn(K_, N, device="cuda", generator=g) * 0.05).bfloat16()
+    bias, res = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((N,), (M, N)))
+    h, ln = torch.randn(M, K_, device="cuda", generator=g).bfloat16(), torch.ones(K_, device="cuda").bfloat16()
+    x = native.rms_norm_fwd(h, ln, 1e-5)[0]                      # the kernel before, which does not write the weights
+    out = native.gemm_skinny(x, w, bias=bias, residual=res, weights_ready=True)
+    act = native.gemm_skinny(x, w, swiglu=True, weights_ready=True) if N % 16 == 0 else None
+    torch.cuda.synchronize()
+    _lib.check_status()
+    prod = x.double() @ w.double()
+    ref = prod + bias.double() + res.double()
+    # as test_skinny_gemm: one rounding to bf16 and an fp32 sum of K_ products of size 0.05; silu is good to some 1e-6 of its terms
+    sums = 0.05 * K_ * 2 ** -22
+    assert (out.double() - ref).abs().le(ref.abs() * 2 ** -8 + sums).all()
+    if act is not None:
+        gate, up = prod.chunk(2, 1)
+        ref = torch.nn.functional.silu(gate) * up
+        assert (act.double() - ref).abs().le(ref.abs() * 2 ** -8 + 1e-3).all()
+
+
 @pytest.mark.parametrize("M,H,N", [(1, 512, 1536), (17, 2048, 5120), (128, 4096, 1024)])
 def test_skinny_gemm_behind_the_kernels_of_a_decode_step(M, H, N):
     """As a decode step launches it, with weights fetched ahead of the wait: the norm kernel just before writes x and the residual,

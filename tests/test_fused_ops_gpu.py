@@ -311,6 +311,27 @@ def test_gemm_residual_epilogue(M, N, K, act):
         assert ((y.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-3 + (2 ** -6 if act else 0)).all()
 
 
+@pytest.mark.parametrize("M,N,K,width", [(2331, 5120, 512, 256), (2048, 2600, 8200, 512), (2048, 2840, 8200, 512)])
+@pytest.mark.parametrize("with_bias", [False, True])
+@pytest.mark.parametrize("round_product", [False, True])
+def test_gemm_residual_epilogue_of_wide_tiles(M, N, K, width, with_bias, round_product):
+    """Tiles of 256 columns, and of 512 whose last one has no second half or a partly filled one; a residual with its own row stride."""
+    from paddle_b200.ops import _lib, native
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _lib.kernels().pd_gemm_2cta_tile_n_at(M, N, K, 1, 0) == width
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w, b, wide = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((M, K), (K, N), (N,), (M, N + 16)))
+    res = wide[:, 8:N + 8]
+    y = native.gemm_epilogue(x, w, b if with_bias else None, residual=res, round_product=round_product)
+    _lib.check_status()
+    h = x.double() @ w.double() + (b.double() if with_bias else 0)
+    # the tensor cores cut off when they add: K / 16 steps lose up to 2^-23 of a running sum below 5 sqrt(K); bias and residual are added
+    # in fp32; one rounding to bf16, with round_product one of the product before it
+    tol = K / 16 * 5 * K ** 0.5 * 2 ** -23 + 2 ** -22 * h.abs() + (2 ** -8 * h.abs() if round_product else 0)
+    ref = h + res.double()
+    assert ((y.double() - ref).abs() <= 2 ** -8 * (ref.abs() + tol) + tol).all()
+
+
 @pytest.mark.parametrize("tokens", [1, 295, 296, 1203])
 @pytest.mark.parametrize("heads,D", [(1, 128), (5, 128), (33, 128), (9, 64), (3, 2048)])
 def test_rope_whole_blocks_and_teams(tokens, heads, D):
