@@ -1,13 +1,14 @@
 // Two-SM (cta_group::2) variant of the persistent bf16 GEMM for sm_100a:  C[M,N] (=|+=) op(A)[M,K] * op(B)[K,N]
 //
-// A cluster of two CTAs (one SM pair) owns a 256 x TN output tile, TN = 256, for products whose tiles all run at once 128, for deep
-// ones 512 in two accumulators of 256 columns (tile_n below).  CTA r of the pair loads rows [128 r, 128 r + 128) of the A tile and columns [TN / 2 r, TN / 2 (r + 1)) of the
-// B tile into ITS OWN shared memory (plain per-CTA TMA loads, no cluster multicast), so with TN = 256 every k-block costs each SM
-// 32 KB of shared-memory fill (six stages; 24 KB and eight stages with TN = 128) instead of the 48 KB of the 128 x 256
-// single-CTA tile, and the tensor core reads half of B from the partner SM.  One thread of the leader CTA (cluster rank 0; its MMA
-// warp stays converged and predicates the instruction: with a one-lane branch the same tiles took 4 to 12 % longer, 4096 x 11008 x
-// 4096 with B transposed 258 against 228 us) issues tcgen05.mma.cta_group::2 (M = 256, N = TN, K = 16); the accumulator rows
-// 0-127 live in the leader's TMEM, rows 128-255 in the partner's, and each CTA's four epilogue warps drain their own half.
+// A cluster of two CTAs (one SM pair) owns a 256 x TN output tile: TN = 256, for products whose tiles all run at once 128, for deep ones
+// 512 (tile_n below).  An accumulator holds ACC_N = min(TN, 256) columns; a 512-column tile is two of them side by side.  CTA r of the
+// pair loads rows [128 r, 128 r + 128) of the A tile and, of each accumulator's columns, [ACC_N / 2 r, ACC_N / 2 (r + 1)) of the B tile
+// into ITS OWN shared memory (plain per-CTA TMA loads, no cluster multicast); the tensor core reads the other half of B from the
+// partner SM.  A 64-deep K block fills 32 KB of each SM with TN = 256 (six stages), 24 KB with 128 (eight stages), 48 KB with 512
+// (four stages: A 16 KB, B 16 KB for each accumulator); the 128 x 256 single-CTA tile takes 48 KB.  One thread of the leader CTA
+// (cluster rank 0; its MMA warp stays converged and predicates the instruction: with a one-lane branch the same tiles took 4 to 12 %
+// longer, 4096 x 11008 x 4096 with B transposed 258 against 228 us) issues tcgen05.mma.cta_group::2 (M = 256, N = ACC_N, K = 16); the
+// accumulator rows 0-127 live in the leader's TMEM, rows 128-255 in the partner's, and each CTA's four epilogue warps drain their half.
 //
 // Barriers (all waits bounded, see sm100_prims.cuh):
 //   full[s]   leader only, 1 arrival + transaction bytes of BOTH CTAs (the partner's TMA loads complete on the
@@ -30,7 +31,7 @@ constexpr int TILE_M = 256;
 constexpr int A_STAGE_BYTES = BM * BK * 2;        // 16 KB
 constexpr int C_CHUNK_BYTES = BM * 128;
 constexpr int NUM_THREADS = 192;
-// TN: columns of the pair's tile, 512, 256 or 128; each CTA holds half of the B tile
+// TN: columns of the pair's tile, 512, 256 or 128; each CTA holds half of the columns of each accumulator
 constexpr int stages(int tn) { return tn == 512 ? 4 : (tn == 256 ? 6 : 8); }
 constexpr int b_stage_bytes(int tn) { return tn / 2 * BK * 2; }
 constexpr int smem_bytes(int tn) { return stages(tn) * (A_STAGE_BYTES + b_stage_bytes(tn)) + 2 * C_CHUNK_BYTES + 1024 + 256; }
@@ -553,8 +554,8 @@ static int tile_n(int M, int N, int K, int splits, int max_ctas) {
 }  // namespace gemm2
 }  // namespace pd
 
-// Columns of the tiles that pd_gemm_bf16_2cta works in.
-PD_EXPORT int pd_gemm_2cta_tile_n(int M, int N, int splits, int max_ctas) { return pd::gemm2::tile_n(M, N, 0, splits, max_ctas); }   // shallow ones
+// Columns of the tiles that pd_gemm_bf16_2cta works in: for K below 8192, and for any K.
+PD_EXPORT int pd_gemm_2cta_tile_n(int M, int N, int splits, int max_ctas) { return pd::gemm2::tile_n(M, N, 0, splits, max_ctas); }
 PD_EXPORT int pd_gemm_2cta_tile_n_at(int M, int N, int K, int splits, int max_ctas) { return pd::gemm2::tile_n(M, N, K, splits, max_ctas); }
 
 // Same contract as pd_gemm_bf16 / pd_gemm_bf16_splitk (gemm_sm100.cu); splits = 1 for the plain form.

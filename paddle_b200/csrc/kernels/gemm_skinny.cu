@@ -140,10 +140,12 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 4) {
     if (lane == 0) {
-      // Large weights pass through the L2 without pushing out x and the cached keys (us, normal / first to leave: 64 rows 5120 x 15360
-      // 28.8 / 27.3, 5120 x 32000 52.1 / 49.9, 13824 x 5120 29.7 / 28.9, 128 rows 4096 x 22016 38.8 / 37.0, one row 28.8 / 28.6).  A model
-      // whose weights are all smaller than this may fit the L2 (126 MB) from token to token, so those stay: with 40 MB as the line one
-      // layer of 1024 and its 65 MB head took 49.1 instead of 47.2.
+      // Large weights pass through the L2 without pushing out x and the cached keys.  us, normal / first to leave: behind other kernels of a
+      // step 64 rows 5120 x 15360 28.8 / 27.3, 5120 x 32000 52.1 / 49.9, 128 rows 4096 x 22016 38.8 / 37.0, one row 28.8 / 28.6.  The line
+      // is a matrix of which no second fits the L2 (126 MB).  Two in turn, 64 rows: 48 MB 15.3 / 15.0, 62 MB 18.6 / 18.5, 68 MB 19.5 /
+      // 19.3, 76 MB 19.5 / 19.0, 86 MB 20.5 / 19.8; twelve: 14.9 / 14.8, 17.0 / 16.8, 17.7 / 17.5, 18.1 / 17.8, 19.4 / 19.0; one row 0 to
+      // 2 %.  So below it there is little to gain, and a small model, whose weights may stay from token to token, has something to lose:
+      // one layer of 1024 and its 65 MB head 47.2 / 49.1.
       const bool pass_through = static_cast<int64_t>(p.K) * p.N * 2 >= (int64_t(72) << 20);
       const uint64_t policy = l2_evict_first();
       prefetch_tmap(&tmW);
