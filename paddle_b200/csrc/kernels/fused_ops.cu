@@ -106,10 +106,10 @@ constexpr int RNW_THREADS = 128;   // small CTAs, so that their turnover does no
 // residual the bf16-rounded sum is what gets normalised (and stored when residual_out is given).
 // Lane l adds up the vectors l, l + 32, l + 64, ... of a row one after the other and the lanes are added at the end, whatever the number
 // of warps: a warp holds consecutive groups of 32 vectors and goes on from the sums of the warp before it.
-// A warp for each row needed 128 registers: 16 warps an SM, each a chain of loads, sums and stores of a whole row; now some 32 are
-// active, with shorter chains.  us, one warp a row / this: 4096 x 4096 18.9 / 14.8, with residual 37.0 / 24.9, 16384 x 4096 with
-// residual 119 / 84 (82 at the copy rate), 2331 x 5120 14.5 / 12.5, 8192 x 2048 16.7 / 14.6; two warps for 4096 and 5120 16.6, 33.1,
-// 103, 14.5.
+// A warp for each row needed 128 registers: 14 of 64 warps an SM were active, each a chain of loads, sums and stores of a whole row.  Now
+// 57 are, as rows no more than before, but each is done in a quarter of the time.  us, one warp a row / this: 4096 x 4096 18.9 / 14.7, with
+// residual 37.0 / 24.9, 16384 x 4096 with residual 119 / 84 (82 at the copy rate), 65536 x 4096 232 / 197 (184 with every warp's sum from
+// zero), 2331 x 5120 14.5 / 12.5, 8192 x 2048 16.7 / 14.6; two warps for 4096 and 5120 16.6, 33.1, 103, -, 14.5.
 constexpr int rnw_warps(int nv) { return nv <= 8 ? 2 : 4; }
 template <typename WT, int NV, bool RES>
 __global__ void __launch_bounds__(RNW_THREADS) rms_norm_fwd_rows_kernel(

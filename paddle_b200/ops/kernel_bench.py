@@ -226,7 +226,8 @@ def bench_decode(args, timer, hbm, tf):
 
 
 def bench_moe(args, timer, hbm, tf):
-    """Grouped block-scaled fp8 expert GEMM (all experts in one launch) against the per-expert bf16 GEMM loop."""
+    """Grouped block-scaled fp8 expert GEMM (all experts in one launch) against the per-expert bf16 GEMM loop, and the bf16 weight
+    gradients of all experts, added into fp32."""
     from . import native
     E, M, K_, N = (4, 8192, 4096, 8192) if args.small else (8, 16384, 4096, 28672)
     per = M // E
@@ -241,6 +242,9 @@ def bench_moe(args, timer, hbm, tf):
     tq = timer(lambda: native.fp8_quant_1x128(x), args.iters)
     rec = dict(op="grouped_gemm_fp8", E=E, M=M, K=K_, N=N, ms=t, tflops=fl / t / 1e9, frac_of_measured_bf16_peak=fl / t / 1e9 / tf,
                act_quant_ms=tq)
+    acc = torch.zeros(E, K_, N, device="cuda")
+    tw = timer(lambda: native.gemm_grouped_tn(x, out, [per] * E, acc, accumulate=True), args.iters)
+    rec.update(wgrad_ms=tw, wgrad_tflops=fl / tw / 1e9)
     if not args.no_baseline:
         def loop():
             for e in range(E):
